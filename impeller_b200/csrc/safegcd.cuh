@@ -5,25 +5,31 @@
 // points), so variable time is fine.
 //
 // The method (D. J. Bernstein and B.-Y. Yang, "Fast constant-time gcd
-// computation and modular inversion", 2019) keeps an odd f (initially the
-// modulus p), a g (initially the input x) and an integer eta, and applies
-// divsteps: with g odd and eta < 0, (f, g) <- (g, (g - f) / 2) and eta <-
-// -eta - 1; with g odd and eta >= 0, g <- (g + f) / 2 and eta <- eta - 1;
-// with g even, g <- g / 2 and eta <- eta - 1.  g reaches 0 with f = +-1.
-// Divsteps look only at the low bits of f and g, so 30 of them at a time run
-// on the low 32-bit words alone, collecting a 2x2 transition matrix
-// T = [u v; q r] with 2^30 (f', g') = T (f, g); the full-width numbers are
-// then updated once per batch.  Beside f and g the method carries d and e
-// with d x = f and e x = g (mod p); they take the same matrix, divided by
-// 2^30 modulo p, so at the end x^-1 = +-d.
+// computation and modular inversion", 2019, in the form that starts at
+// delta = 1/2) keeps an odd f (initially the modulus p), a g (initially the
+// input x) and zeta = -(delta + 1/2), and applies divsteps: with g odd and
+// zeta < 0, (f, g) <- (g, (g - f) / 2) and zeta <- -zeta - 2; with g odd and
+// zeta >= 0, g <- (g + f) / 2 and zeta <- zeta - 1; with g even, g <- g / 2
+// and zeta <- zeta - 1.  g reaches 0 with f = +-1.  Divsteps look only at the
+// low bits of f and g, so 30 of them at a time run on the low 32-bit words
+// alone, collecting a 2x2 transition matrix T = [u v; q r] with
+// 2^30 (f', g') = T (f, g); the full-width numbers are then updated once per
+// batch.  Beside f and g the method carries d and e with d x = f and e x = g
+// (mod p); they take the same matrix, divided by 2^30 modulo p, so at the end
+// x^-1 = +-d.
 //
-// Inside a batch, runs of even steps are taken at once (count of trailing
-// zeros), and consecutive odd steps that keep f are merged: while eta stays
-// non-negative for the next `limit` steps, adding w f with
-// w = -g / f mod 2^limit clears `limit` low bits of g, which is what those
-// steps would do one by one.  |u| + |v| <= 2^30 and |q| + |r| <= 2^30 after a
-// batch, so the matrix fits 32-bit signed integers (intermediate values wrap
+// The 30 steps of a batch are straight-line code on masks (18 instructions a
+// step): taking runs of even steps at once and merging odd steps needs fewer
+// instructions for one input, but its loop depends on the input, so the lanes
+// of a warp wait for the longest, and its count of trailing zeros and Newton
+// steps are one long chain.  |u| + |v| <= 2^30 and |q| + |r| <= 2^30 after a
+// batch, so the matrix fits 32-bit signed integers (the words wrap
 // consistently modulo 2^32).
+//
+// d and e are not reduced between batches: an update takes a pair bounded by
+// B p to one bounded by (B + 1/2) p (the multiple of p that makes the sum
+// divisible by 2^30 is below 2^29 in magnitude), which the limbs hold through
+// the last batch; one reduction at the end.
 //
 // Multi-precision numbers are signed radix-2^30: limbs 0..L-2 in [0, 2^30),
 // the top limb signed.  Written for host and device so that the host build
@@ -54,65 +60,42 @@ struct Trans {
     int32_t u, v, q, r;
 };
 
-SG_HD int ctz32(uint32_t x) {
-#if defined(__CUDA_ARCH__)
-    return __ffs((int)x) - 1;
-#else
-    return __builtin_ctz(x);
-#endif
-}
-
-// Limb count for an N-word (32-bit) modulus: the values stay below 2p in
-// magnitude, plus a sign.
+// Limb count for an N-word (32-bit) modulus: room for the unreduced d and e
+// (magnitude below 2^5 p for 8 words, 2^6 p for 12; the fields' moduli leave
+// two and three bits of their words free) and a sign.
 SG_CX int limbs_for(int N) { return (32 * N + 2 + 29) / 30; }
 
 // Upper bound of batches: Bernstein-Yang's bound of (49 d + 57) / 17 divsteps
-// for d-bit inputs, in batches of 30, plus one.
+// for d-bit inputs (the delta = 1/2 form needs fewer), in batches of 30, plus
+// one.
 SG_CX int max_batches(int N) { return ((49 * 32 * N + 57) / 17 + 29) / 30 + 1; }
 
-// 30 divsteps on the low words of f (odd) and g; returns the new eta.
-SG_HD int divsteps30(int eta, uint32_t f, uint32_t g, Trans &t) {
+// 30 divsteps on the low words of f (odd) and g; returns the new zeta.
+SG_HD int divsteps30(int zeta, uint32_t f, uint32_t g, Trans &t) {
     uint32_t u = 1, v = 0, q = 0, r = 1;
-    int i = 30;
-    for (;;) {
-        const int z = ctz32(g | (0xffffffffu << i));  // even steps, at most i
-        g >>= z;
-        u <<= z;
-        v <<= z;
-        eta -= z;
-        i -= z;
-        if (i == 0) break;
-        // f and g odd
-        if (eta < 0) {
-            uint32_t x;
-            eta = -eta;
-            x = f;
-            f = g;
-            g = 0u - x;
-            x = u;
-            u = q;
-            q = 0u - x;
-            x = v;
-            v = r;
-            r = 0u - x;
-        }
-        const int limit = (eta + 1) > i ? i : (eta + 1);
-        const uint32_t m = 0xffffffffu >> (32 - limit);
-        // f^-1 mod 2^32: (3f) xor 2 is right to 5 bits, each Newton step doubles that
-        uint32_t fi = (3u * f) ^ 2u;
-        fi *= 2u - f * fi;
-        fi *= 2u - f * fi;
-        fi *= 2u - f * fi;
-        const uint32_t w = (0u - g * fi) & m;
-        g += f * w;
-        q += u * w;
-        r += v * w;
+#if defined(__CUDA_ARCH__)
+#pragma unroll 10
+#endif
+    for (int i = 0; i < 30; i++) {
+        const uint32_t odd = 0u - (g & 1u);
+        const uint32_t swap = odd & (uint32_t)(zeta >> 31);
+        // (x ^ swap) & odd, less swap: 0, x or -x
+        const uint32_t df = (f ^ swap) & odd, du = (u ^ swap) & odd, dv = (v ^ swap) & odd;
+        f ^= (f ^ g) & swap;
+        u ^= (u ^ q) & swap;
+        v ^= (v ^ r) & swap;
+        g = (g + df - swap) >> 1;
+        q = q + du - swap;
+        r = r + dv - swap;
+        u <<= 1;
+        v <<= 1;
+        zeta = (zeta ^ (int)swap) - 1;
     }
     t.u = (int32_t)u;
     t.v = (int32_t)v;
     t.q = (int32_t)q;
     t.r = (int32_t)r;
-    return eta;
+    return zeta;
 }
 
 // (f, g) <- T (f, g) / 2^30 (exact).
@@ -142,38 +125,30 @@ SG_HD bool s30_neg(const S30<L> &x) {
     return x.v[L - 1] < 0;
 }
 
-// x >= p for x >= 0
+// s x + k p for s = +-1 and a small k, the limbs renormalised
 template <int L>
-SG_HD bool s30_geq(const S30<L> &x, const S30<L> &p) {
-#pragma unroll
-    for (int i = L - 1; i >= 0; i--)
-        if (x.v[i] != p.v[i]) return x.v[i] > p.v[i];
-    return true;
-}
-
-// x += s * p for s = +-1, renormalising the limbs
-template <int L>
-SG_HD void s30_add_mul(S30<L> &x, const S30<L> &p, int32_t s) {
+SG_HD S30<L> s30_mul_add(const S30<L> &x, int32_t s, const S30<L> &p, int32_t k) {
+    S30<L> y;
     int64_t c = 0;
 #pragma unroll
     for (int i = 0; i < L - 1; i++) {
-        c += (int64_t)x.v[i] + (int64_t)s * p.v[i];
-        x.v[i] = (int32_t)(c & M30);
+        c += (int64_t)s * x.v[i] + (int64_t)k * p.v[i];
+        y.v[i] = (int32_t)(c & M30);
         c >>= 30;
     }
-    x.v[L - 1] = (int32_t)(c + x.v[L - 1] + (int64_t)s * p.v[L - 1]);
+    y.v[L - 1] = (int32_t)(c + (int64_t)s * x.v[L - 1] + (int64_t)k * p.v[L - 1]);
+    return y;
 }
 
-// (d, e) <- T (d, e) / 2^30 mod p, for d, e in [0, p); results in [0, p).
-// pinv = p^-1 mod 2^30.
+// (d, e) <- T (d, e) / 2^30 mod p, unreduced.  pinv = p^-1 mod 2^30.
 template <int L>
 SG_HD void update_de(S30<L> &d, S30<L> &e, const Trans &t, const S30<L> &p, uint32_t pinv) {
     const int64_t u = t.u, v = t.v, q = t.q, r = t.r;
     int64_t cd = u * d.v[0] + v * e.v[0];
     int64_t ce = q * d.v[0] + r * e.v[0];
-    // md, me in [0, 2^30) make the low 30 bits of cd + md p and ce + me p zero
-    const int64_t md = (int64_t)((0u - (uint32_t)cd * pinv) & M30);
-    const int64_t me = (int64_t)((0u - (uint32_t)ce * pinv) & M30);
+    // md, me in [-2^29, 2^29) make the low 30 bits of cd + md p and ce + me p zero
+    const int64_t md = (int32_t)((0u - (uint32_t)cd * pinv) << 2) >> 2;
+    const int64_t me = (int32_t)((0u - (uint32_t)ce * pinv) << 2) >> 2;
     cd += md * p.v[0];
     ce += me * p.v[0];
     cd >>= 30;
@@ -189,11 +164,6 @@ SG_HD void update_de(S30<L> &d, S30<L> &e, const Trans &t, const S30<L> &p, uint
     }
     d.v[L - 1] = (int32_t)cd;
     e.v[L - 1] = (int32_t)ce;
-    // (u d + v e + m p) / 2^30 lies in [-p, 2p): one correction each way
-    if (s30_neg(d)) s30_add_mul(d, p, 1);
-    else if (s30_geq(d, p)) s30_add_mul(d, p, -1);
-    if (s30_neg(e)) s30_add_mul(e, p, 1);
-    else if (s30_geq(e, p)) s30_add_mul(e, p, -1);
 }
 
 template <int L>
@@ -260,20 +230,24 @@ SG_HD void inverse(const uint32_t *x, const uint32_t *pw, uint32_t *out) {
 #pragma unroll
     for (int k = 0; k < N; k++) out[k] = 0;
     if (s30_is_zero(g)) return;
-    int eta = -1;
+    // |d| <= (1 + max_batches / 2) p < K p at the end
+    constexpr int K = N == 8 ? 16 : 32;
+    static_assert(1 + max_batches(N) / 2 < K, "the last batch's d");
+    int zeta = -1;
 #pragma unroll 1
     for (int b = 0; b < max_batches(N); b++) {
         Trans t;
-        eta = divsteps30(eta, (uint32_t)f.v[0] | ((uint32_t)f.v[1] << 30),
-                         (uint32_t)g.v[0] | ((uint32_t)g.v[1] << 30), t);
+        zeta = divsteps30(zeta, (uint32_t)f.v[0] | ((uint32_t)f.v[1] << 30),
+                          (uint32_t)g.v[0] | ((uint32_t)g.v[1] << 30), t);
         update_fg(f, g, t);
         update_de(d, e, t, p, pinv);
         if (s30_is_zero(g)) {
-            // f = +-1: x^-1 = +-d
-            if (s30_neg(f) && !s30_is_zero(d)) {
-                S30<L> n = p;
-                s30_add_mul(n, d, -1);
-                d = n;
+            // f = +-1: x^-1 = +-d; into [0, 2 K p), then below p
+            d = s30_mul_add(d, s30_neg(f) ? -1 : 1, p, K);
+#pragma unroll 1
+            for (int k = K; k; k >>= 1) {
+                const S30<L> r = s30_mul_add(d, 1, p, -k);
+                if (!s30_neg(r)) d = r;
             }
             from_s30<L, N>(d, out);
             return;
