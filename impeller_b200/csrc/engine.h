@@ -55,13 +55,18 @@ struct PlanLayout {
     size_t o_recb, o_recp, o_parts, o_parts_s, o_wres, o_long, o_carry, o_results;
     // two-level sort
     size_t o_cnt, o_coff, o_ccur, o_ctiles, o_centry, o_cfine, o_segs, o_binseg, o_nsegs, o_seghist, o_segcur;
+    // pairwise affine levels: odd and even levels' points, last level's bucket starts
+    size_t o_pair_odd, o_pair_even, o_pair_scratch, o_pair_off;
     size_t bytes;
 };
 
 class Plan {
   public:
     // Every MSM reads points[table_base + (w / n_windows) * table_stride + i].
-    static bool build(Plan &p, int device, const std::vector<MsmShape> &shapes);
+    // pairs: the plan may add points pairwise in affine form before the
+    // accumulation, where that is faster; it then takes more scratch (the
+    // levels' points).
+    static bool build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool pairs = false);
     // Whether a plan of these shapes would sort its entries with the
     // two-level counting sort (fast) rather than the per-entry atomic sort
     // that build() falls back to for very large batches.
@@ -128,6 +133,7 @@ class Plan {
     u64 max_entries = 0;
     u32 accum_blocks = 0, accum_block = 256;
     u32 nparts = 0, long_cap = 0;
+    u32 pair_levels = 0;  // k_affine_pairs levels before the accumulation
     u32 hist_grid_x = 1;
     // two-level sort (msd) or per-entry atomic bucket sort
     bool msd = false;

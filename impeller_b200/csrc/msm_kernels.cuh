@@ -28,6 +28,7 @@
 // the canonical affine result runs on the device.
 #pragma once
 
+#include "affine_pairs.cuh"
 #include "bn254.cuh"
 
 namespace impeller {
@@ -625,6 +626,9 @@ struct AccumArgs {
     u32 *buckets;        // XYZZ, 32 u32 each, indexed by global bucket
     u32 *rec_bucket;     // 2 per thread
     u32 *rec_point;      // 2 per thread, XYZZ
+    // After k_affine_pairs (pair_state not null and nonzero): the last
+    // level's points, in bucket order; `offsets` are that level's.
+    const u32 *pair_state, *pair_odd, *pair_even;
 };
 
 template <class C>
@@ -703,12 +707,17 @@ __global__ void __launch_bounds__(AccumShape<C>::threads, AccumShape<C>::per_sm)
     u32 bbeg = a.offsets[b], bend = a.offsets[b + 1];
     u32 seg_end = min(bend, end);
 
+    // entries of the sort, or the pairwise levels' points in order
+    const u32 levels = a.pair_state ? *a.pair_state : 0;
+    const u32 *const points = levels ? (levels & 1u ? a.pair_odd : a.pair_even) : a.points;
+    const auto entry = [&](u32 pos) { return levels ? pos << 1 : a.entries[pos]; };
+
     XyzzT<FQ> acc = xyzz_identity<FQ>();
     bool fresh = true;
-    AffineT<FQ> nxt = load_entry_point<C>(a.points, a.entries[start]);
+    AffineT<FQ> nxt = load_entry_point<C>(points, entry(start));
     for (u32 pos = start; pos < end; pos++) {
         AffineT<FQ> q = nxt;
-        if (pos + 1 < end) nxt = load_entry_point<C>(a.points, a.entries[pos + 1]);
+        if (pos + 1 < end) nxt = load_entry_point<C>(points, entry(pos + 1));
         // One mixed-addition code path for every entry: a bucket start only
         // picks the value the addition starts from (lanes of a warp start
         // buckets at different entries, and a second inlined addition on
