@@ -59,6 +59,7 @@ struct Config {
     bool debug;
     u32 curve;
     u32 PW, XW;  // affine and XYZZ point words
+    bool glv = false;  // BN254 without window tables: scalars split by the endomorphism
 };
 
 bool make_config(unsigned window_size, unsigned target_window, int debug, Config &cfg, u32 curve = CURVE_BN254) {
@@ -140,7 +141,11 @@ u32 stream_chunks(u64 len) { return (u32)stream_bounds(len).size() - 1; }
 // parts > 1: each part is a chunk, in one of two buffer stages.
 constexpr u32 PART_STAGES = 2;
 
+// The caller's window without tables sets only the digit width (every digit
+// window has its own bucket set), so a split scalar takes the nearest width
+// that suits its halves.
 std::vector<MsmShape> group_shapes(const Config &cfg, u32 M, u32 n, u32 part_len) {
+    if (cfg.glv) return std::vector<MsmShape>(M, MsmShape{n, split_window(cfg.c), 0, 0, 0, cfg.curve, part_len});
     std::vector<MsmShape> s(M, MsmShape{n, cfg.c, cfg.n_windows, part_len, 0, cfg.curve});
     return s;
 }
@@ -260,7 +265,7 @@ DevicePlans &device_plans(int device) {
 constexpr size_t PLAN_CACHE_CAP = 32;
 
 Plan *cached_plan(DevicePlans &D, int device, const Config &cfg, u32 M, u32 n, u32 stride) {
-    std::vector<u32> key{cfg.c, cfg.n_windows, M, n, stride, cfg.curve};
+    std::vector<u32> key{cfg.c, cfg.n_windows, M, n, stride, cfg.curve, cfg.glv ? 1u : 0u};
     auto it = D.plans.find(key);
     if (it != D.plans.end()) {
         it->second.gen = D.gen;
@@ -521,6 +526,12 @@ cudaError_t impeller_msm_cfg_curve(unsigned int curve, unsigned int window_size,
     if (parts == 0 || batch_per_run == 0) {
         set_error("msm: parts and batch_per_run must be at least 1");
         return cudaErrorInvalidValue;
+    }
+    if (curve == CURVE_BN254 && cfg.n_tables == 1) {
+        // the halves' digits and the images' indices have to fit 32 bits
+        const u64 per_card = (len + num_cards - 1) / num_cards, part = (per_card + parts - 1) / parts;
+        cfg.glv = 2 * part < (1ull << 31) &&
+                  2ull * ((128 + split_window(cfg.c) - 1) / split_window(cfg.c)) * batch_per_run * part < 0xffffffffull;
     }
     std::vector<CardLayout> layouts(num_cards);
     for (u32 i = 0; i < num_cards; i++) {

@@ -45,6 +45,11 @@ static constexpr u32 PAIR_BLOCK = 128;
 static constexpr u32 PAIR_MAX_LEVELS = 6;
 static constexpr u64 PAIR_SCRATCH_MAX = 16ull << 30;  // bytes of the first level's points
 static constexpr u32 PAIR_NONE = 0xffffffffu;
+
+// Where points come from: entries of the sort, entries among which indices
+// from phi_base on stand for images under the endomorphism, or the previous
+// level's points in order.
+enum : int { FROM_ENTRIES = 0, FROM_IMAGES = 1, FROM_LEVEL = 2 };
 template <class C>
 struct PairShape {
     static constexpr u32 per_sm = C::XW == 32 ? PAIR_BLOCKS_PER_SM : PAIR_BLOCKS_PER_SM_BLS;
@@ -71,6 +76,8 @@ struct PairArgs {
     const u32 *points;   // level 0: the point array; else the previous level's points
     u32 *out;
     unsigned char *scratch;  // PairShape::block_bytes per block
+    const u32 *phi;          // level 0: the images' abscissae, for entries of index phi_base + i
+    u32 phi_base;
     const u32 *used;         // number of levels that run (k_pair_plan)
     u32 *next_unit;          // zero at launch
 };
@@ -135,7 +142,7 @@ struct PairWalk {
         window = offsets[min(b + (threadIdx.x & 31u), nb)];
     }
     // s: ascending over lanes and calls, below the last bucket's end
-    template <bool FIRST>
+    template <int FROM>
     __device__ __forceinline__ uint2 at(u32 s, u32 lane) {
         u32 mine = NOT_FOUND, beg = 0, end = 0;
         for (;;) {
@@ -163,15 +170,37 @@ struct PairWalk {
         if (j >= cnt) return make_uint2(PAIR_NONE, PAIR_NONE);
         const u32 i = (u32)level_start(beg, mine, level) + j;
         const bool two = j + 1 < cnt;
-        if constexpr (FIRST) return make_uint2(entries[i], two ? entries[i + 1] : PAIR_NONE);
+        if constexpr (FROM != FROM_LEVEL) return make_uint2(entries[i], two ? entries[i + 1] : PAIR_NONE);
         else return make_uint2(i, two ? i + 1 : PAIR_NONE);
     }
     static constexpr u32 NOT_FOUND = 0xffffffffu;
 };
 
-template <class C, bool FIRST>
-__device__ __forceinline__ const u32 *pair_point(const u32 *points, u32 e) {
-    return points + (size_t)(FIRST ? e >> 1 : e) * C::PW;
+// Where an entry's coordinates lie.  Index phi_base + i is the image of point
+// i under the endomorphism (beta x, y): its abscissa lies in phi.
+template <class C, bool IMAGES>
+__device__ __forceinline__ void entry_coordinates(const u32 *points, u32 e, const u32 *phi, u32 phi_base,
+                                                  const u32 *&px, const u32 *&py) {
+    u32 i = e >> 1;
+    if constexpr (IMAGES) {
+        const bool image = i >= phi_base;
+        if (image) i -= phi_base;
+        py = points + (size_t)i * C::PW + C::Fq::N;
+        px = image ? phi + (size_t)i * C::Fq::N : py - C::Fq::N;
+    } else {
+        px = points + (size_t)i * C::PW;
+        py = px + C::Fq::N;
+    }
+}
+
+template <class C, int FROM>
+__device__ __forceinline__ void pair_coordinates(const PairArgs &a, u32 e, const u32 *&px, const u32 *&py) {
+    if constexpr (FROM != FROM_LEVEL) {
+        entry_coordinates<C, FROM == FROM_IMAGES>(a.points, e, a.phi, a.phi_base, px, py);
+    } else {
+        px = a.points + (size_t)e * C::PW;
+        py = px + C::Fq::N;
+    }
 }
 
 // Asynchronous copy of the leading CH 16-byte chunks of 32 points, one per
@@ -180,17 +209,22 @@ __device__ __forceinline__ const u32 *pair_point(const u32 *points, u32 e) {
 // that misses the TLB costs the same for one 32-byte sector as for the whole
 // point: 38 G random requests/s over tables of 0.5 GB and more on B200, so
 // lane-wise loads of a 64-byte point, two requests, reach 19 G points/s.)
-template <class C, bool FIRST, u32 CH>
-__device__ __forceinline__ void stage_points(const u32 *points, u32 e, u32 dst, u32 lane) {
+template <class C, int FROM, u32 CH>
+__device__ __forceinline__ void stage_points(const PairArgs &a, u32 e, u32 dst, u32 lane) {
 #pragma unroll
     for (u32 j = 0; j < CH; j++) {
         const u32 c = lane + 32 * j, pt = c / CH, ch = c % CH;
         const u32 ee = __shfl_sync(0xffffffffu, e, pt);
         // no copy where there is no point: copies of one stand-in would all
         // queue at its L2 slice
-        if (ee != PAIR_NONE) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + pt * PairShape<C>::point_bytes + ch * 16),
-                     "l"(pair_point<C, FIRST>(points, ee) + ch * 4)
-                     : "memory");
+        if (ee != PAIR_NONE) {
+            const u32 *px, *py;
+            pair_coordinates<C, FROM>(a, ee, px, py);
+            const u32 *from = ch < C::Fq::N / 4 ? px + ch * 4 : py + ch * 4 - C::Fq::N;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + pt * PairShape<C>::point_bytes + ch * 16),
+                         "l"(from)
+                         : "memory");
+        }
     }
 }
 
@@ -248,10 +282,10 @@ __device__ __forceinline__ bool pair_identity(const Fe<F> &y) {
     return y.l[0] == 0 && fe_is_zero_canonical(y);
 }
 
-template <class C, bool FIRST>
-__device__ __forceinline__ Fe<typename C::Fq> pair_y(const u32 *point, u32 e) {
-    const Fe<typename C::Fq> y = fe_load<typename C::Fq>(point + C::Fq::N);
-    return FIRST && (e & 1u) ? fe_neg(y) : y;
+template <class C, int FROM>
+__device__ __forceinline__ Fe<typename C::Fq> pair_y(const u32 *py, u32 e) {
+    const Fe<typename C::Fq> y = fe_load<typename C::Fq>(py);
+    return FROM != FROM_LEVEL && (e & 1u) ? fe_neg(y) : y;
 }
 
 // One level.  A tile is 128 x kk consecutive output slots, 32 x kk of them a
@@ -259,7 +293,7 @@ __device__ __forceinline__ Fe<typename C::Fq> pair_y(const u32 *point, u32 e) {
 // multiplies its pairs' denominators together (the products before each go to
 // the block's scratch), one warp inverts the 128 totals, and each lane goes
 // back through its pairs.  Blocks take tiles from a counter.
-template <class C, bool FIRST>
+template <class C, int FROM>
 __global__ void __launch_bounds__(PAIR_BLOCK, PairShape<C>::per_sm) k_affine_pairs(PairArgs a) {
     using FQ = typename C::Fq;
     using S = PairShape<C>;
@@ -307,22 +341,22 @@ __global__ void __launch_bounds__(PAIR_BLOCK, PairShape<C>::per_sm) k_affine_pai
             PairWalk walk(a, s0);
             auto look = [&](u32 k) {
                 const u32 s = s0 + 32 * k + lane;
-                uint2 e = walk.at<FIRST>(min(s, total - 1), lane);
+                uint2 e = walk.at<FROM>(min(s, total - 1), lane);
                 if (s >= s1) e = make_uint2(PAIR_NONE, PAIR_NONE);
                 return e;
             };
             // slot inputs are looked up two iterations ahead, their points copied one ahead
             uint2 e = look(0), next = make_uint2(PAIR_NONE, PAIR_NONE);
-            stage_points<C, FIRST, XCH>(a.points, e.x, stage, lane);
-            stage_points<C, FIRST, XCH>(a.points, e.y, stage + SECOND, lane);
+            stage_points<C, FROM, XCH>(a, e.x, stage, lane);
+            stage_points<C, FROM, XCH>(a, e.y, stage + SECOND, lane);
             stage_commit();
             if (n > 1) next = look(1);
 #pragma unroll 1
             for (u32 k = 0; k < n; k++) {
                 if (k + 1 < n) {
                     const u32 at = stage + ((k + 1) & 1u) * S::stage_bytes;
-                    stage_points<C, FIRST, XCH>(a.points, next.x, at, lane);
-                    stage_points<C, FIRST, XCH>(a.points, next.y, at + SECOND, lane);
+                    stage_points<C, FROM, XCH>(a, next.x, at, lane);
+                    stage_points<C, FROM, XCH>(a, next.y, at + SECOND, lane);
                 }
                 stage_commit();
                 uint2 next2 = make_uint2(PAIR_NONE, PAIR_NONE);
@@ -334,8 +368,10 @@ __global__ void __launch_bounds__(PAIR_BLOCK, PairShape<C>::per_sm) k_affine_pai
                     Fe<FQ> d = fe_sub(fe_load<FQ>(p + SECOND / 4), fe_load<FQ>(p));
                     if (pair_zero(d)) {
                         bool dbl;
-                        d = pair_equal_x(pair_y<C, FIRST>(pair_point<C, FIRST>(a.points, e.x), e.x),
-                                         pair_y<C, FIRST>(pair_point<C, FIRST>(a.points, e.y), e.y), dbl);
+                        const u32 *px, *py1, *py2;
+                        pair_coordinates<C, FROM>(a, e.x, px, py1);
+                        pair_coordinates<C, FROM>(a, e.y, px, py2);
+                        d = pair_equal_x(pair_y<C, FROM>(py1, e.x), pair_y<C, FROM>(py2, e.y), dbl);
                     }
                     plane_store<FQ>(my_pre, plane, 32 * k, run);
                     run = fe_mul(run, d);
@@ -354,8 +390,8 @@ __global__ void __launch_bounds__(PAIR_BLOCK, PairShape<C>::per_sm) k_affine_pai
         __syncthreads();
         if (n) {
             uint2 e = my_src[32 * (n - 1)], next = n > 1 ? my_src[32 * (n - 2)] : e;
-            stage_points<C, FIRST, PCH>(a.points, e.x, stage + ((n - 1) & 1u) * S::stage_bytes, lane);
-            stage_points<C, FIRST, PCH>(a.points, e.y, stage + ((n - 1) & 1u) * S::stage_bytes + SECOND, lane);
+            stage_points<C, FROM, PCH>(a, e.x, stage + ((n - 1) & 1u) * S::stage_bytes, lane);
+            stage_points<C, FROM, PCH>(a, e.y, stage + ((n - 1) & 1u) * S::stage_bytes + SECOND, lane);
             if (e.y != PAIR_NONE) stage_product<C>(my_pre + 32 * (n - 1), stage + ((n - 1) & 1u) * S::stage_bytes + PRODUCT, lane);
             stage_commit();
 #pragma unroll 1
@@ -364,8 +400,8 @@ __global__ void __launch_bounds__(PAIR_BLOCK, PairShape<C>::per_sm) k_affine_pai
                 if (k > 1) next2 = my_src[32 * (k - 2)];
                 if (k) {
                     const u32 at = stage + ((k - 1) & 1u) * S::stage_bytes;
-                    stage_points<C, FIRST, PCH>(a.points, next.x, at, lane);
-                    stage_points<C, FIRST, PCH>(a.points, next.y, at + SECOND, lane);
+                    stage_points<C, FROM, PCH>(a, next.x, at, lane);
+                    stage_points<C, FROM, PCH>(a, next.y, at + SECOND, lane);
                     if (next.y != PAIR_NONE) stage_product<C>(my_pre + 32 * (k - 1), at + PRODUCT, lane);
                 }
                 stage_commit();
@@ -377,11 +413,11 @@ __global__ void __launch_bounds__(PAIR_BLOCK, PairShape<C>::per_sm) k_affine_pai
                     Fe<FQ> d = fe_sub(fe_load<FQ>(p2), fe_load<FQ>(p1));
                     bool dbl = false;
                     const bool same = pair_zero(d);
-                    if (same) d = pair_equal_x(pair_y<C, FIRST>(p1, e.x), pair_y<C, FIRST>(p2, e.y), dbl);
+                    if (same) d = pair_equal_x(pair_y<C, FROM>(p1 + FQ::N, e.x), pair_y<C, FROM>(p2 + FQ::N, e.y), dbl);
                     const uint4 *pp = reinterpret_cast<const uint4 *>(stage_ptr + (k & 1u) * S::stage_bytes + PRODUCT);
                     const Fe<FQ> w = fe_mul(inv, plane_load<FQ>(pp, 32, lane));  // 1 / d
                     inv = fe_mul(inv, d);
-                    const Fe<FQ> y1 = pair_y<C, FIRST>(p1, e.x), y2 = pair_y<C, FIRST>(p2, e.y);
+                    const Fe<FQ> y1 = pair_y<C, FROM>(p1 + FQ::N, e.x), y2 = pair_y<C, FROM>(p2 + FQ::N, e.y);
                     Fe<FQ> num = fe_sub(y2, y1);
                     const Fe<FQ> x1 = fe_load<FQ>(p1), x2 = fe_load<FQ>(p2);
                     if (dbl) {
@@ -400,7 +436,7 @@ __global__ void __launch_bounds__(PAIR_BLOCK, PairShape<C>::per_sm) k_affine_pai
                     }
                 } else if (e.x != PAIR_NONE) {
                     r.x = fe_load<FQ>(p1);
-                    r.y = pair_y<C, FIRST>(p1, e.x);
+                    r.y = pair_y<C, FROM>(p1 + FQ::N, e.x);
                 } else {
                     r.x = r.y = fe_zero<FQ>();  // unused slot: the identity
                 }

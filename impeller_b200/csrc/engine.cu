@@ -54,6 +54,17 @@ u32 digit_windows(u32 c, u32 curve) {
             kern<Bn254><<<(grid), (block), (smem), (st)>>>(__VA_ARGS__);               \
     } while (0)
 
+// Launch a digit-recoding kernel for the plan's curve and scalars.
+#define DIGIT_LAUNCH(curve_id, images, kern, grid, block, smem, st, ...)               \
+    do {                                                                               \
+        if ((curve_id) == CURVE_BLS12381)                                              \
+            kern<Bls12381, false><<<(grid), (block), (smem), (st)>>>(__VA_ARGS__);     \
+        else if (images)                                                               \
+            kern<Bn254, true><<<(grid), (block), (smem), (st)>>>(__VA_ARGS__);         \
+        else                                                                           \
+            kern<Bn254, false><<<(grid), (block), (smem), (st)>>>(__VA_ARGS__);        \
+    } while (0)
+
 int sm_count(int device) {
     static std::mutex mu;
     static std::map<int, int> cache;
@@ -68,6 +79,17 @@ int sm_count(int device) {
 
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
+// Digits per scalar and bucket sets of a shape.
+static void shape_windows(const MsmShape &s, u32 &digits, u32 &sets) {
+    if (s.phi_base) {
+        sets = glv::windows(s.c);
+        digits = 2 * sets;
+    } else {
+        digits = digit_windows(s.c, s.curve);
+        sets = (s.n_windows == 0 || s.n_windows > digits) ? digits : s.n_windows;
+    }
+}
+
 // The sort-path rule of Plan::build, from the shapes alone.  Each MSM's
 // buckets start on a multiple of FINE, so every coarse bin belongs to one
 // MSM, and the count matrix holds, per MSM, its bins times its tiles of
@@ -78,13 +100,15 @@ bool Plan::two_level_sort(const std::vector<MsmShape> &shapes) {
     u32 wmax = 1;
     for (const MsmShape &s : shapes) {
         if (s.c < 3 || s.c > 31) return false;
-        wmax = std::max(wmax, digit_windows(s.c, s.curve));
+        u32 W, nw;
+        shape_windows(s, W, nw);
+        wmax = std::max(wmax, W);
     }
     const u32 tile = std::max(32u, std::min(1024u, (STAGE_ENTRIES / wmax) & ~31u));
     u64 stiles = 0, cells = 0;
     for (const MsmShape &s : shapes) {
-        const u32 W = digit_windows(s.c, s.curve);
-        const u32 nw = (s.n_windows == 0 || s.n_windows > W) ? W : s.n_windows;
+        u32 W, nw;
+        shape_windows(s, W, nw);
         nb = align_up(nb, FINE);
         const u64 b0 = nb / FINE;
         nb += (u64)nw << (s.c - 1);
@@ -131,18 +155,28 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
     std::vector<WinDesc> wins;
     u64 nb = 0, entries = 0;
     u32 nmax = 0;
+    p.phi_base = p.phi_points = 0;
     for (u32 m = 0; m < p.M; m++) {
         const MsmShape &s = shapes[m];
         if (s.c < 3 || s.c > 31) {
             set_error("window size must be in [3, 31]");
             return false;
         }
-        const u32 W = digit_windows(s.c, p.curve);
-        const u32 nw = (s.n_windows == 0 || s.n_windows > W) ? W : s.n_windows;
+        u32 W, nw;
+        shape_windows(s, W, nw);
         const u32 n_tables = (W + nw - 1) / nw;
+        const u32 stride = s.phi_base ? s.phi_base : s.table_stride;
         const u64 B = 1ull << (s.c - 1);
-        const u64 vmax = (u64)s.table_base + (u64)(n_tables - 1) * s.table_stride + s.n;
-        if (n_tables > 1 && s.table_stride < s.n) {
+        const u64 vmax = (u64)s.table_base + (u64)(n_tables - 1) * stride + s.n;
+        if (s.phi_base && (p.curve != CURVE_BN254 || s.table_base || (p.phi_base && p.phi_base != s.phi_base))) {
+            set_error("endomorphism images need BN254, table 0 and one base index");
+            return false;
+        }
+        if (s.phi_base) {
+            p.phi_base = s.phi_base;
+            p.phi_points = std::max(p.phi_points, s.n);
+        }
+        if (n_tables > 1 && stride < s.n) {
             set_error("table stride smaller than the MSM size");
             return false;
         }
@@ -157,7 +191,8 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
         d.c = s.c;
         d.n_logical = W;
         d.n_windows = nw;
-        d.table_stride = s.table_stride;
+        d.table_stride = stride;
+        d.glv = s.phi_base ? 1u : 0u;
         d.bucket_base = (u32)nb;
         d.win_base = (u32)wins.size();
         d.table_base = s.table_base;
@@ -344,6 +379,7 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
                                                                 : PairShape<Bn254>::per_sm * PairShape<Bn254>::block_bytes)
                                            : 0);
     lo.o_pair_off = take(p.pair_levels ? (size_t)(p.nb + 2 + PAIR_MAX_LEVELS) * 4 : 0);
+    lo.o_phi = take((size_t)p.phi_points * 32);
     lo.o_buckets = take((size_t)p.nb * XB);
     lo.o_recb = take((size_t)2 * T * 4);
     lo.o_recp = take((size_t)2 * T * XB);
@@ -366,7 +402,7 @@ Plan::~Plan() {
 
 // sort (10 kernels two-level, 6 per-entry) + accumulate, 2 fixups, reduce,
 // one per reduction-tree level, final
-u32 Plan::launches() const { return (msd ? 10u : 6u) + (pair_levels ? pair_levels + 1u : 0u) + 5u + (u32)tree_first.size() - 1u; }
+u32 Plan::launches() const { return (msd ? 10u : 6u) + (pair_levels ? pair_levels + 2u : 0u) + (phi_points ? 1u : 0u) + 5u + (u32)tree_first.size() - 1u; }
 
 const char *Plan::phase_name(int i) {
     static const char *names[NPHASE] = {"tables", "histogram", "scan", "scatter",
@@ -472,8 +508,10 @@ template <class C>
 static cudaError_t launch_pair_levels(int device, u32 curve, u32 levels, PairArgs pa, u32 *odd, u32 *even,
                                       u32 *offsets, u32 *state, cudaStream_t st) {
     constexpr size_t smem = PairShape<C>::smem;
-    CK(cudaFuncSetAttribute(k_affine_pairs<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CK(cudaFuncSetAttribute(k_affine_pairs<C, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr int IMAGES = C::XW == 32 ? FROM_IMAGES : FROM_ENTRIES;
+    CK(cudaFuncSetAttribute(k_affine_pairs<C, FROM_ENTRIES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(cudaFuncSetAttribute(k_affine_pairs<C, IMAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(cudaFuncSetAttribute(k_affine_pairs<C, FROM_LEVEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     pa.sms = (u32)sm_count(device);
     pa.used = state;
     k_pair_plan<<<std::max(1u, std::min((pa.nb + 256) / 256, pa.sms * 8)), 256, 0, st>>>(
@@ -484,12 +522,30 @@ static cudaError_t launch_pair_levels(int device, u32 curve, u32 levels, PairArg
         pa.level = l;
         pa.out = l & 1u ? even : odd;
         pa.next_unit = state + 1 + l;
-        if (l == 0) k_affine_pairs<C, true><<<grid, PAIR_BLOCK, smem, st>>>(pa);
-        else k_affine_pairs<C, false><<<grid, PAIR_BLOCK, smem, st>>>(pa);
+        if (l) k_affine_pairs<C, FROM_LEVEL><<<grid, PAIR_BLOCK, smem, st>>>(pa);
+        else if (pa.phi_base != NONE) k_affine_pairs<C, IMAGES><<<grid, PAIR_BLOCK, smem, st>>>(pa);
+        else k_affine_pairs<C, FROM_ENTRIES><<<grid, PAIR_BLOCK, smem, st>>>(pa);
         CK_LAUNCH("k_affine_pairs");
         pa.points = pa.out;
     }
     return cudaSuccess;
+}
+
+// k_accumulate for the plan's curve, bucket start (carry: streamed chunks) and
+// source of points.
+template <int FROM>
+static void launch_accumulate(u32 curve, bool carry, bool images, u32 grid, u32 block, const AccumArgs &aa,
+                              cudaStream_t st) {
+    if (curve == CURVE_BLS12381) {
+        if (carry) k_accumulate<Bls12381, START_CARRY, FROM><<<grid, block, 0, st>>>(aa);
+        else k_accumulate<Bls12381, ACCUM_START_BLS, FROM><<<grid, block, 0, st>>>(aa);
+    } else if (images) {
+        if (carry) k_accumulate<Bn254, START_CARRY, FROM_IMAGES><<<grid, block, 0, st>>>(aa);
+        else k_accumulate<Bn254, START_CONVERT, FROM_IMAGES><<<grid, block, 0, st>>>(aa);
+    } else {
+        if (carry) k_accumulate<Bn254, START_CARRY, FROM><<<grid, block, 0, st>>>(aa);
+        else k_accumulate<Bn254, START_CONVERT, FROM><<<grid, block, 0, st>>>(aa);
+    }
 }
 
 // k_coarse_scatter (kernel 0) and k_seg_scatter (kernel 1) stage entries in
@@ -551,7 +607,7 @@ cudaError_t Plan::run_front(void *scratch, const u32 *points, cudaStream_t st, b
         k_zero_words<<<1, 256, 0, st>>>(cnt + ncnt, cnt_pad - ncnt, p.longl, 1);
         CK_LAUNCH("k_zero_words");
         MARK(1);
-        CURVE_LAUNCH(curve, k_coarse_count, sort_tiles, SORT_BLOCK, nbins * 4, st, sa);
+        DIGIT_LAUNCH(curve, phi_points, k_coarse_count, sort_tiles, SORT_BLOCK, nbins * 4, st, sa);
         CK_LAUNCH("k_coarse_count");
         MARK(2);
         k_scan_reduce<<<cscan_tiles, SCAN_BLOCK, 0, st>>>(cnt, ctiles);
@@ -584,7 +640,7 @@ cudaError_t Plan::run_front(void *scratch, const u32 *points, cudaStream_t st, b
         MARK(1);
 
         dim3 hgrid(hist_grid_x, M);
-        CURVE_LAUNCH(curve, k_histogram, hgrid, 256, 0, st, p.desc, p.counts);
+        DIGIT_LAUNCH(curve, phi_points, k_histogram, hgrid, 256, 0, st, p.desc, p.counts);
         CK_LAUNCH("k_histogram");
         MARK(2);
         k_scan_reduce<<<ntiles, SCAN_BLOCK, 0, st>>>(p.counts, p.tiles);
@@ -594,20 +650,26 @@ cudaError_t Plan::run_front(void *scratch, const u32 *points, cudaStream_t st, b
         k_scan_down<<<ntiles, SCAN_BLOCK, 0, st>>>(p.counts, p.tiles, p.offsets, p.cursor, nb, ntiles);
         CK_LAUNCH("k_scan_down");
         MARK(3);
-        CURVE_LAUNCH(curve, k_scatter, hgrid, 256, 0, st, p.desc, p.cursor, p.entries);
+        DIGIT_LAUNCH(curve, phi_points, k_scatter, hgrid, 256, 0, st, p.desc, p.cursor, p.entries);
         CK_LAUNCH("k_scatter");
         MARK(4);
     }
 
     if (points_ready) CK(cudaStreamWaitEvent(st, points_ready, 0));
     u32 *const buckets = bucket_out ? bucket_out : p.buckets;
+    u32 *const phi = reinterpret_cast<u32 *>(static_cast<unsigned char *>(scratch) + layout.o_phi);
+    const u32 phi_from = phi_points ? phi_base : NONE;
+    if (phi_points) {
+        k_images<<<std::min((phi_points + 127) / 128, (u32)sm_count(device) * 16), 128, 0, st>>>(points, phi_points, phi);
+        CK_LAUNCH("k_images");
+    }
     const u32 *offsets = p.offsets;
-    AccumArgs aa{p.entries, offsets, nb, points, buckets, p.recb, p.recp, nullptr, nullptr, nullptr};
+    AccumArgs aa{p.entries, offsets, nb, points, buckets, p.recb, p.recp, nullptr, nullptr, nullptr, phi, phi_from};
     if (pair_levels) {
         unsigned char *sb = static_cast<unsigned char *>(scratch);
         u32 *odd = reinterpret_cast<u32 *>(sb + layout.o_pair_odd), *even = reinterpret_cast<u32 *>(sb + layout.o_pair_even);
         u32 *state = p.level_offsets + nb + 1;
-        const PairArgs pa{p.offsets, nb, 0, 0, p.entries, points, nullptr, sb + layout.o_pair_scratch, nullptr, nullptr};
+        const PairArgs pa{p.offsets, nb, 0, 0, p.entries, points, nullptr, sb + layout.o_pair_scratch, phi, phi_from, nullptr, nullptr};
         cudaError_t e = curve == CURVE_BLS12381
                             ? launch_pair_levels<Bls12381>(device, curve, pair_levels, pa, odd, even, p.level_offsets, state, st)
                             : launch_pair_levels<Bn254>(device, curve, pair_levels, pa, odd, even, p.level_offsets, state, st);
@@ -617,13 +679,10 @@ cudaError_t Plan::run_front(void *scratch, const u32 *points, cudaStream_t st, b
         aa.pair_odd = odd;
         aa.pair_even = even;
     }
-    if (bucket_out) {
-        if (curve == CURVE_BLS12381) k_accumulate<Bls12381, START_CARRY><<<accum_blocks, accum_block, 0, st>>>(aa);
-        else k_accumulate<Bn254, START_CARRY><<<accum_blocks, accum_block, 0, st>>>(aa);
-    } else if (curve == CURVE_BLS12381) {
-        k_accumulate<Bls12381, ACCUM_START_BLS><<<accum_blocks, accum_block, 0, st>>>(aa);
-    } else {
-        k_accumulate<Bn254, START_CONVERT><<<accum_blocks, accum_block, 0, st>>>(aa);
+    launch_accumulate<FROM_ENTRIES>(curve, bucket_out != nullptr, phi_points != 0, accum_blocks, accum_block, aa, st);
+    if (pair_levels) {
+        CK_LAUNCH("k_accumulate");
+        launch_accumulate<FROM_LEVEL>(curve, bucket_out != nullptr, false, accum_blocks, accum_block, aa, st);
     }
     CK_LAUNCH("k_accumulate");
     MARK(5);
@@ -813,6 +872,22 @@ u32 curve_window(u32 c, u32 curve) {
     return c < 16 ? c + 1 : c - 1;
 }
 
+// Plain windows on BN254 cut the two 128-bit halves of a scalar (glv.cuh).  A
+// width that leaves the halves' top digit only a few bits sends every scalar
+// into few of that window's buckets (n = 100003, c = 15, 7 top bits: 0.11 ms
+// of fixups), so the choice moves to the nearest width that does not: 8, 13
+// and 16 divide 128 or nearly so, 10 leaves 8 bits of 10, 19 leaves 14, 22
+// leaves 18.  The window table was measured on whole scalars; measured on the
+// halves the moved choices are the best widths at 2^10, 2^12, 2^14, 2^18,
+// 2^20 and 2^22 points, and 2 % off at 100003.
+u32 split_window(u32 c) {
+    static const u32 widths[] = {8, 10, 13, 16, 19, 22};
+    u32 best = c;
+    for (u32 w : widths)
+        if ((w > c ? w - c : c - w) <= 1) best = w;
+    return best;
+}
+
 // Window of the resident tables the table recommends for MSMs of n points
 // (0: plain windows are faster at that size).
 u32 table_window(u64 n) {
@@ -840,7 +915,8 @@ u32 impeller::ctx_set_base(const impeller_ctx *ctx, u32 c) {
 u32 impeller::ctx_window(const impeller_ctx *ctx, u64 n) {
     const u32 ct = table_window(n);
     if (ct && ctx_set_base(ctx, ct) != NONE) return ct;
-    return curve_window(default_window(n), ctx->curve);
+    const u32 c = default_window(n);
+    return ctx->curve == CURVE_BN254 ? split_window(c) : curve_window(c, ctx->curve);
 }
 
 static cudaError_t ctx_reserve(impeller_ctx *ctx, size_t bytes, cudaStream_t st) {
@@ -860,7 +936,11 @@ static cudaError_t ctx_reserve(impeller_ctx *ctx, size_t bytes, cudaStream_t st)
 MsmShape impeller::ctx_shape(const impeller_ctx *ctx, u32 n, u32 c) {
     const u32 base = ctx_set_base(ctx, c);
     if (base != NONE) return MsmShape{n, c, 1, (u32)ctx->len, base, ctx->curve};
-    return MsmShape{n, c, 0, 0, 0, ctx->curve};
+    MsmShape s{n, c, 0, 0, 0, ctx->curve};
+    const u64 have = ctx->tables ? ctx->tables_points : ctx->len;
+    if (ctx->curve == CURVE_BN254 && have + n < (1ull << 31) && 2ull * glv::windows(c) * n < 0xffffffffull)
+        s.phi_base = (u32)have;
+    return s;
 }
 
 const u32 *impeller::ctx_point_base(const impeller_ctx *ctx) { return ctx->tables ? ctx->tables : ctx->points; }

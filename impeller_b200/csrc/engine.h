@@ -35,6 +35,10 @@ struct MsmShape {
     u32 table_stride;  // points per window table (used when n_windows < digit windows)
     u32 table_base;    // point index of this MSM's table 0
     u32 curve;         // CURVE_BN254 or CURVE_BLS12381
+    // BN254, plain windows: nonzero splits the scalars by the endomorphism
+    // (glv.cuh); the images of the points take the virtual indices from here
+    // on (at least the point array's length; the same for every MSM of a plan).
+    u32 phi_base = 0;
 };
 
 // Signed-digit windows of width c for the curve's scalars: the fewest that
@@ -44,6 +48,7 @@ struct MsmShape {
 u32 digit_windows(u32 c, u32 curve = CURVE_BN254);
 u32 default_window(u64 n);  // autotune table (or the cost model)
 u32 table_window(u64 n);    // tables window the autotune table recommends (0: none)
+u32 split_window(u32 c);    // c moved off widths whose top digit of a split BN254 scalar is short
 u32 curve_window(u32 c, u32 curve);  // c moved off windows that need an extra digit window on the curve
 
 // Device property cache.
@@ -57,6 +62,7 @@ struct PlanLayout {
     size_t o_cnt, o_coff, o_ccur, o_ctiles, o_centry, o_cfine, o_segs, o_binseg, o_nsegs, o_seghist, o_segcur;
     // pairwise affine levels: odd and even levels' points, last level's bucket starts
     size_t o_pair_odd, o_pair_even, o_pair_scratch, o_pair_off;
+    size_t o_phi;  // the points' images under the endomorphism: x
     size_t bytes;
 };
 
@@ -134,6 +140,7 @@ class Plan {
     u32 accum_blocks = 0, accum_block = 256;
     u32 nparts = 0, long_cap = 0;
     u32 pair_levels = 0;  // k_affine_pairs levels before the accumulation
+    u32 phi_base = 0, phi_points = 0;  // endomorphism images: first virtual index, points (0: none)
     u32 hist_grid_x = 1;
     // two-level sort (msd) or per-entry atomic bucket sort
     bool msd = false;

@@ -30,6 +30,7 @@
 
 #include "affine_pairs.cuh"
 #include "bn254.cuh"
+#include "glv.cuh"
 
 namespace impeller {
 
@@ -55,6 +56,8 @@ struct MsmDesc {
     u32 win_base;        // global index of physical window 0
     u32 table_base;      // index of this MSM's table 0 in the point array
     u32 entry_base;      // first digit slot of this MSM (sum of n * n_logical of the earlier MSMs)
+    u32 glv;             // scalars split by the endomorphism: n_windows digits of either half, the
+                         // second half's points at table_stride (the images' virtual indices)
 };
 
 // One physical window of one MSM (bucket reduction unit).
@@ -81,8 +84,9 @@ struct WinDesc {
 // a digit costs one 64-bit shift, and the window and table indices advance
 // by counting instead of dividing.  Every lane runs the same windows (the
 // count depends only on c and n_logical).
-template <class FR, class Emit>
-__device__ __forceinline__ void for_each_digit(const Fe<FR> &v, u32 c, u32 n_logical, u32 n_windows, Emit &&emit) {
+template <int LIMBS, class Emit>
+__device__ __forceinline__ void for_each_digit(const u32 (&limbs)[LIMBS], u32 c, u32 n_logical, u32 n_windows,
+                                               Emit &&emit) {
     const u32 mask = (1u << c) - 1u, half = 1u << (c - 1);
     u64 buf = 0;
     u32 nbits = 0, carry = 0, w = 0, pw = 0, table = 0;
@@ -102,8 +106,8 @@ __device__ __forceinline__ void for_each_digit(const Fe<FR> &v, u32 c, u32 n_log
         }
     };
 #pragma unroll
-    for (int k = 0; k < FR::N; k++) {
-        buf |= (u64)v.l[k] << nbits;
+    for (int k = 0; k < LIMBS; k++) {
+        buf |= (u64)limbs[k] << nbits;
         nbits += 32;
         while (nbits >= c && w + 1 < n_logical) {
             step((u32)buf & mask, false);
@@ -118,12 +122,35 @@ __device__ __forceinline__ void for_each_digit(const Fe<FR> &v, u32 c, u32 n_log
     step((u32)buf & mask, true);
 }
 
+// The digits of an MSM's scalar: of the scalar itself, or of its two halves
+// (MsmDesc::glv), the second one's as table 1.  GLV: the plan may hold such
+// MSMs (a kernel for both is 10 % slower where none does).
+template <class C, bool GLV, class Emit>
+__device__ __forceinline__ void for_each_digit(const MsmDesc &d, const Fe<typename C::Fr> &v, Emit &&emit) {
+    if constexpr (GLV) {
+        if (d.glv) {
+            u32 k[2][4], neg[2];
+            glv::split(v.l, k[0], neg[0], k[1], neg[1]);
+#pragma unroll 1
+            for (u32 h = 0; h < 2; h++) {
+                const u32 l[4] = {h ? k[1][0] : k[0][0], h ? k[1][1] : k[0][1], h ? k[1][2] : k[0][2],
+                                  h ? k[1][3] : k[0][3]};
+                const u32 n = h ? neg[1] : neg[0];
+                for_each_digit<4>(l, d.c, d.n_windows, d.n_windows,
+                                  [&](u32 pw, u32, u32 mag, u32 sign) { emit(pw, h, mag, sign ^ n); });
+            }
+            return;
+        }
+    }
+    for_each_digit<C::Fr::N>(v.l, d.c, d.n_logical, d.n_windows, emit);
+}
+
 // Lanes of a warp whose digits hit the same bucket share one atomic: heavy
 // buckets (the top window in a shared bucket set, the 0 / 1 / small scalars of
 // witness-like inputs) would otherwise serialize on a handful of addresses.
 // Every lane of the warp runs the same number of windows, so the match is
 // always taken with the full warp present.
-template <class C>
+template <class C, bool GLV>
 __global__ void k_histogram(const MsmDesc *__restrict__ descs, u32 *__restrict__ counts) {
     const MsmDesc d = descs[blockIdx.y];
     const u32 B = 1u << (d.c - 1);
@@ -134,7 +161,7 @@ __global__ void k_histogram(const MsmDesc *__restrict__ descs, u32 *__restrict__
         const bool live = i < d.n;
         const Fe<typename C::Fr> v = live ? fe_from_mont<typename C::Fr>(fe_load<typename C::Fr>(d.scalars + 8ull * i))
                                           : fe_zero<typename C::Fr>();
-        for_each_digit(v, d.c, d.n_logical, d.n_windows, [&](u32 pw, u32, u32 mag, u32) {
+        for_each_digit<C, GLV>(d, v, [&](u32 pw, u32, u32 mag, u32) {
             const u32 key = mag ? d.bucket_base + pw * B + mag - 1 : NONE;
             const u32 peers = __match_any_sync(0xffffffffu, key);
             if (key != NONE && lane == __ffs(peers) - 1) atomicAdd(&counts[key], (u32)__popc(peers));
@@ -142,7 +169,7 @@ __global__ void k_histogram(const MsmDesc *__restrict__ descs, u32 *__restrict__
     }
 }
 
-template <class C>
+template <class C, bool GLV>
 __global__ void k_scatter(const MsmDesc *__restrict__ descs, u32 *__restrict__ cursor, u32 *__restrict__ entries) {
     const MsmDesc d = descs[blockIdx.y];
     const u32 B = 1u << (d.c - 1);
@@ -153,7 +180,7 @@ __global__ void k_scatter(const MsmDesc *__restrict__ descs, u32 *__restrict__ c
         const bool live = i < d.n;
         const Fe<typename C::Fr> v = live ? fe_from_mont<typename C::Fr>(fe_load<typename C::Fr>(d.scalars + 8ull * i))
                                           : fe_zero<typename C::Fr>();
-        for_each_digit(v, d.c, d.n_logical, d.n_windows, [&](u32 pw, u32 table, u32 mag, u32 sign) {
+        for_each_digit<C, GLV>(d, v, [&](u32 pw, u32 table, u32 mag, u32 sign) {
             const u32 key = mag ? d.bucket_base + pw * B + mag - 1 : NONE;
             const u32 peers = __match_any_sync(0xffffffffu, key);
             const u32 leader = __ffs(peers) - 1;
@@ -266,7 +293,7 @@ __device__ __forceinline__ void sort_tile(const SortArgs &a, u32 tile, u32 &m, u
     end = min(start + a.tile_scalars, a.descs[m].n);
 }
 
-template <class C>
+template <class C, bool GLV>
 __global__ void __launch_bounds__(SORT_BLOCK) k_coarse_count(SortArgs a) {
     extern __shared__ u32 hist[];  // nbins
     u32 m, start, end;
@@ -286,7 +313,7 @@ __global__ void __launch_bounds__(SORT_BLOCK) k_coarse_count(SortArgs a) {
         const Fe<typename C::Fr> v = live ? fe_from_mont<typename C::Fr>(fe_load<typename C::Fr>(d.scalars + 8ull * i))
                                           : fe_zero<typename C::Fr>();
         u32 *kw = kp + (i - start);
-        for_each_digit(v, d.c, d.n_logical, d.n_windows, [&](u32 pw, u32, u32 mag, u32 sign) {
+        for_each_digit<C, GLV>(d, v, [&](u32 pw, u32, u32 mag, u32 sign) {
             u32 key = NONE;
             if (mag) {
                 key = d.bucket_base + pw * B + mag - 1;
@@ -629,6 +656,10 @@ struct AccumArgs {
     // After k_affine_pairs (pair_state not null and nonzero): the last
     // level's points, in bucket order; `offsets` are that level's.
     const u32 *pair_state, *pair_odd, *pair_even;
+    // Abscissae of the points' images under the endomorphism (k_images);
+    // entries of index phi_base + i take theirs from here.
+    const u32 *phi;
+    u32 phi_base;
 };
 
 template <class C>
@@ -636,6 +667,25 @@ __device__ __forceinline__ AffineT<typename C::Fq> load_entry_point(const u32 *_
     AffineT<typename C::Fq> q = affine_load<typename C::Fq>(points + (size_t)(e >> 1) * C::PW);
     if (e & 1u) q.y = fe_neg(q.y);
     return q;
+}
+
+template <class C>
+__device__ __forceinline__ AffineT<typename C::Fq> load_entry_point(const u32 *__restrict__ points, u32 e,
+                                                                    const u32 *__restrict__ phi, u32 phi_base) {
+    const u32 *px, *py;
+    entry_coordinates<C, true>(points, e, phi, phi_base, px, py);
+    AffineT<typename C::Fq> q;
+    q.x = fe_load<typename C::Fq>(px);
+    q.y = fe_load<typename C::Fq>(py);
+    if (e & 1u) q.y = fe_neg(q.y);
+    return q;
+}
+
+// x of the points' images under the endomorphism: beta x.
+__global__ void k_images(const u32 *__restrict__ points, u32 n, u32 *__restrict__ phi) {
+    const Fq beta = {GLV_BETA};
+    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        fe_store(phi + 8ull * i, fe_mul<FqP>(fe_load<FqP>(points + 16ull * i), beta));
 }
 
 // Thread t owns entries [t*L, min((t+1)*L, E)), L = ceil(E / T).
@@ -682,9 +732,15 @@ enum : int { START_CONVERT = 0, START_IDENTITY = 1, START_CARRY = 2 };
 #define ACCUM_START_BLS START_IDENTITY
 #endif
 
-template <class C, int START = START_CONVERT>
+// FROM: the entries' points (FROM_ENTRIES, FROM_IMAGES) or, after
+// k_affine_pairs, the last level's.  Where the device decides whether levels
+// run (k_pair_plan), both kernels are launched and one returns at once: a
+// kernel that picked at run time was 4 % slower on BN254.
+template <class C, int START = START_CONVERT, int FROM = FROM_ENTRIES>
 __global__ void __launch_bounds__(AccumShape<C>::threads, AccumShape<C>::per_sm) k_accumulate(AccumArgs a) {
     using FQ = typename C::Fq;
+    const u32 levels = a.pair_state ? *a.pair_state : 0;
+    if ((FROM == FROM_LEVEL) != (levels != 0)) return;
     const u32 T = gridDim.x * blockDim.x;
     const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
     const u32 E = a.offsets[a.nb];
@@ -707,17 +763,19 @@ __global__ void __launch_bounds__(AccumShape<C>::threads, AccumShape<C>::per_sm)
     u32 bbeg = a.offsets[b], bend = a.offsets[b + 1];
     u32 seg_end = min(bend, end);
 
-    // entries of the sort, or the pairwise levels' points in order
-    const u32 levels = a.pair_state ? *a.pair_state : 0;
-    const u32 *const points = levels ? (levels & 1u ? a.pair_odd : a.pair_even) : a.points;
-    const auto entry = [&](u32 pos) { return levels ? pos << 1 : a.entries[pos]; };
+    const u32 *const points = FROM == FROM_LEVEL ? (levels & 1u ? a.pair_odd : a.pair_even) : a.points;
+    const auto load = [&](u32 pos) {
+        if constexpr (FROM == FROM_LEVEL) return affine_load<FQ>(points + (size_t)pos * C::PW);
+        else if constexpr (FROM == FROM_IMAGES) return load_entry_point<C>(points, a.entries[pos], a.phi, a.phi_base);
+        else return load_entry_point<C>(points, a.entries[pos]);
+    };
 
     XyzzT<FQ> acc = xyzz_identity<FQ>();
     bool fresh = true;
-    AffineT<FQ> nxt = load_entry_point<C>(points, entry(start));
+    AffineT<FQ> nxt = load(start);
     for (u32 pos = start; pos < end; pos++) {
         AffineT<FQ> q = nxt;
-        if (pos + 1 < end) nxt = load_entry_point<C>(points, entry(pos + 1));
+        if (pos + 1 < end) nxt = load(pos + 1);
         // One mixed-addition code path for every entry: a bucket start only
         // picks the value the addition starts from (lanes of a warp start
         // buckets at different entries, and a second inlined addition on
