@@ -77,6 +77,60 @@ int sm_count(int device) {
     return v;
 }
 
+// Scratch memory that outlives one context: freed scratch stays mapped for the
+// next context or batch, so that a new one's first MSM does not wait for the
+// mapping (4 to 5 ms per GB).  At most SCRATCH_KEEP bytes per device stay,
+// and none once the device's last holder is gone.
+static constexpr u64 SCRATCH_KEEP = 6ull << 30;
+
+struct ScratchPool {
+    cudaMemPool_t pool = nullptr;
+    u32 holders = 0;
+};
+static std::mutex g_pool_mu;
+static std::map<int, ScratchPool> g_pools;
+
+cudaError_t scratch_hold(int device) {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    ScratchPool &p = g_pools[device];
+    if (!p.pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        CK(cudaMemPoolCreate(&p.pool, &props));
+        u64 keep = SCRATCH_KEEP;
+        CK(cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+    p.holders++;
+    return cudaSuccess;
+}
+
+void scratch_release(int device) {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    ScratchPool &p = g_pools[device];
+    if (p.holders && --p.holders == 0) {
+        cudaStreamSynchronize(nullptr);  // the frees before this
+        cudaMemPoolTrimTo(p.pool, 0);
+    }
+}
+
+cudaError_t scratch_alloc(void **out, size_t bytes, int device, cudaStream_t st) {
+    cudaMemPool_t pool;
+    {
+        std::lock_guard<std::mutex> g(g_pool_mu);
+        pool = g_pools[device].pool;
+    }
+    cudaError_t e = cudaMallocFromPoolAsync(out, bytes, pool, st);
+    if (e == cudaErrorMemoryAllocation) {
+        // freed pieces may be in the way of a larger one
+        (void)cudaGetLastError();
+        cudaMemPoolTrimTo(pool, 0);
+        e = cudaMallocFromPoolAsync(out, bytes, pool, st);
+    }
+    return e;
+}
+
 static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Digits per scalar and bucket sets of a shape.
@@ -923,10 +977,10 @@ static cudaError_t ctx_reserve(impeller_ctx *ctx, size_t bytes, cudaStream_t st)
     if (bytes <= ctx->scratch_bytes) return cudaSuccess;
     CK(cudaStreamSynchronize(st));
     CK(cudaEventSynchronize(ctx->done));
-    if (ctx->scratch) CK(cudaFree(ctx->scratch));
+    if (ctx->scratch) CK(cudaFreeAsync(ctx->scratch, st));
     ctx->scratch = nullptr;
     ctx->scratch_bytes = 0;
-    CK(cudaMalloc(&ctx->scratch, bytes));
+    CK(scratch_alloc(&ctx->scratch, bytes, ctx->device, st));
     ctx->scratch_bytes = bytes;
     return cudaSuccess;
 }
@@ -1028,6 +1082,8 @@ cudaError_t impeller_ctx_create_curve(impeller_ctx **out, int device, const uint
         ctx->owns = true;
     }
     CK(cudaMalloc(&ctx->d_result, PB));
+    CK(scratch_hold(device));
+    ctx->held = true;
     *out = ctx.release();
     return cudaSuccess;
 }
@@ -1038,7 +1094,8 @@ cudaError_t impeller_ctx_destroy(impeller_ctx *ctx) {
     cudaDeviceSynchronize();
     if (ctx->owns) cudaFree(const_cast<u32 *>(ctx->points));
     if (ctx->tables) cudaFree(ctx->tables);
-    if (ctx->scratch) cudaFree(ctx->scratch);
+    if (ctx->scratch) cudaFreeAsync(ctx->scratch, nullptr);
+    if (ctx->held) scratch_release(ctx->device);
     if (ctx->d_scalars) cudaFree(ctx->d_scalars);
     if (ctx->d_result) cudaFree(ctx->d_result);
     if (ctx->done) cudaEventDestroy(ctx->done);
@@ -1207,6 +1264,8 @@ struct impeller_batch {
     cudaGraph_t g = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaStream_t cap_stream = nullptr;
+    int device = 0;
+    bool held = false;  // of the device's scratch pool
 };
 
 extern "C" {
@@ -1228,16 +1287,27 @@ cudaError_t impeller_batch_create(impeller_batch **out, impeller_ctx *ctx, const
     }
     std::unique_ptr<impeller_batch> b(new impeller_batch());
     b->ctx = ctx;
+    b->device = ctx->device;
     if (!Plan::build(b->plan, ctx->device, shapes, true)) return cudaErrorInvalidValue;
     CK(cudaSetDevice(ctx->device));
-    cudaError_t e = cudaMalloc(&b->scratch, b->plan.scratch_bytes());
+    CK(scratch_hold(ctx->device));
+    b->held = true;
+    cudaError_t e = scratch_alloc(&b->scratch, b->plan.scratch_bytes(), ctx->device, nullptr);
     if (e == cudaErrorMemoryAllocation && b->plan.pair_levels) {
         // no room for the affine levels' points: the plan without them
         (void)cudaGetLastError();
-        if (!Plan::build(b->plan, ctx->device, shapes, false)) return cudaErrorInvalidValue;
-        e = cudaMalloc(&b->scratch, b->plan.scratch_bytes());
+        if (!Plan::build(b->plan, ctx->device, shapes, false)) {
+            scratch_release(ctx->device);
+            return cudaErrorInvalidValue;
+        }
+        e = scratch_alloc(&b->scratch, b->plan.scratch_bytes(), ctx->device, nullptr);
     }
-    CK(e);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // any stream may run the batch
+    if (e != cudaSuccess) {
+        scratch_release(ctx->device);
+        set_error(std::string("impeller_batch_create: scratch: ") + cudaGetErrorString(e));
+        return e;
+    }
     b->graph = (flags & IMPELLER_BATCH_GRAPH) != 0;
     *out = b.release();
     return cudaSuccess;
@@ -1250,7 +1320,8 @@ cudaError_t impeller_batch_destroy(impeller_batch *b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->g) cudaGraphDestroy(b->g);
     if (b->cap_stream) cudaStreamDestroy(b->cap_stream);
-    if (b->scratch) cudaFree(b->scratch);
+    if (b->scratch) cudaFreeAsync(b->scratch, nullptr);
+    if (b->held) scratch_release(b->device);
     delete b;
     return cudaSuccess;
 }

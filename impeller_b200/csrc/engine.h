@@ -181,6 +181,12 @@ class Plan {
     cudaError_t prof_mark(int k, cudaStream_t st);
 };
 
+// Scratch from a per-device pool (engine.cu): stream-ordered like
+// cudaMallocAsync, freed with cudaFreeAsync.  Holders keep freed scratch mapped.
+cudaError_t scratch_hold(int device);
+void scratch_release(int device);
+cudaError_t scratch_alloc(void **out, size_t bytes, int device, cudaStream_t st);
+
 // k_combine: sum `k` XYZZ points in device memory, write canonical affine.
 cudaError_t combine_xyzz(const u32 *d_xyzz, u32 k, u32 *d_out, cudaStream_t stream, u32 curve = CURVE_BN254);
 
@@ -205,6 +211,7 @@ struct impeller_ctx {
     impeller::u32 *d_result = nullptr;
     cudaEvent_t done = nullptr;  // last run that used the scratch
     bool profiling = false;
+    bool held = false;  // of the device's scratch pool
     // Resident window tables: one allocation holding the points (region 0)
     // followed by table sets; the set for window c has W(c) tables of len
     // points, table j = 2^(j*c) * P, starting at point index base.
