@@ -644,19 +644,37 @@ cudaError_t impeller_msm_precompute_cfg_curve(unsigned int curve, unsigned int w
         const u64 cnt = std::min<u64>(per, len - off);
         if (cnt == 0) return cudaSuccess;
         CK(cudaSetDevice(dev));
-        cudaStream_t st = device_stream(dev);
-        const u64 chunk = std::min<u64>(cnt, 1ull << 20);
+        // Chunks alternate between two streams and buffers, so that one
+        // chunk's tables are copied back while the next one is computed.
+        cudaStream_t st[2] = {device_stream(dev, 0), device_stream(dev, 1)};
+        if (!st[0] || !st[1]) {
+            set_error("msm_precompute: could not create a stream");
+            return cudaErrorUnknown;
+        }
+        const u64 chunk = std::min<u64>(cnt, std::min<u64>(1ull << 19, std::max<u64>(1ull << 14, (cnt + 3) / 4)));
+        const u64 buffer = (u64)cfg.n_tables * chunk * PW;
         u32 *d = nullptr;
-        CK(cudaMalloc(&d, (size_t)cfg.n_tables * chunk * PW * 4));
+        CK(cudaMalloc(&d, (size_t)2 * buffer * 4));
         cudaError_t e = cudaSuccess;
-        for (u64 s = 0; s < cnt && e == cudaSuccess; s += chunk) {
+        auto download = [&](u64 s, u32 k) {
             const u64 m = std::min<u64>(chunk, cnt - s);
-            e = cudaMemcpyAsync(d, h_points[0] + (off + s) * PW, m * PW * 4, cudaMemcpyHostToDevice, st);
-            if (e == cudaSuccess) e = precompute_tables(d, m, shift, cfg.n_tables, st, cfg.curve);
             for (u32 t = 1; t < cfg.n_tables && e == cudaSuccess; t++)
-                e = cudaMemcpyAsync(h_points[t] + (off + s) * PW, d + (size_t)t * m * PW, m * PW * 4,
-                                    cudaMemcpyDeviceToHost, st);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+                e = cudaMemcpyAsync(h_points[t] + (off + s) * PW, d + k * buffer + (size_t)t * m * PW, m * PW * 4,
+                                    cudaMemcpyDeviceToHost, st[k]);
+        };
+        u32 k = 0;
+        for (u64 s = 0; s < cnt && e == cudaSuccess; s += chunk, k ^= 1) {
+            const u64 m = std::min<u64>(chunk, cnt - s);
+            u32 *dk = d + k * buffer;
+            // (stream order keeps the buffer's previous chunk ahead of this copy)
+            e = cudaMemcpyAsync(dk, h_points[0] + (off + s) * PW, m * PW * 4, cudaMemcpyHostToDevice, st[k]);
+            if (e == cudaSuccess) e = precompute_tables(dk, m, shift, cfg.n_tables, st[k], cfg.curve);
+            if (s) download(s - chunk, k ^ 1);
+        }
+        if (e == cudaSuccess) download((cnt - 1) / chunk * chunk, k ^ 1);
+        for (cudaStream_t x : st) {
+            const cudaError_t w = cudaStreamSynchronize(x);
+            if (e == cudaSuccess) e = w;
         }
         cudaFree(d);
         if (e != cudaSuccess) set_error(std::string("msm_precompute: ") + cudaGetErrorString(e));

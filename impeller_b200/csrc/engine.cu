@@ -838,15 +838,58 @@ cudaError_t combine_xyzz(const u32 *d_xyzz, u32 k, u32 *d_out, cudaStream_t stre
     return cudaSuccess;
 }
 
+// Window tables of one point per thread: table j = 2^shift (table j - 1).
+// Bound by the integer multiply pipe, so: the doublings run in Jacobian
+// coordinates (812 partial products each on BN254 against XYZZ's 1140), the
+// chain goes on from table to table, and a group of tables shares one divstep
+// inversion (seven products a table to affine form; a Fermat inversion per
+// table was 310).  The host call with 2^17 points and 4 further tables of 52
+// doublings, copies included: 10.6 -> 5.9 ms.
+static constexpr u32 PRECOMPUTE_GROUP = 16;
 template <class C>
-__global__ void k_precompute(u32 *points, u64 n, u32 shift, u32 n_tables) {
+__global__ void __launch_bounds__(128) k_precompute(u32 *points, u64 n, u32 shift, u32 n_tables) {
     using FQ = typename C::Fq;
     const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    XyzzT<FQ> p = xyzz_from_affine(affine_load<FQ>(points + i * C::PW));
-    for (u32 j = 1; j < n_tables; j++) {
-        for (u32 k = 0; k < shift; k++) p = xyzz_dbl(p);
-        affine_store(points + ((u64)j * n + i) * C::PW, xyzz_to_affine(p));
+    const AffineT<FQ> a = affine_load<FQ>(points + i * C::PW);
+    if (affine_is_identity(a)) {
+        AffineT<FQ> zero;
+        zero.x = zero.y = fe_zero<FQ>();
+        for (u32 j = 1; j < n_tables; j++) affine_store(points + ((u64)j * n + i) * C::PW, zero);
+        return;
+    }
+    JacT<FQ> p;
+    p.x = a.x;
+    p.y = a.y;
+    p.z = fe_one<FQ>();
+    Fe<FQ> z[PRECOMPUTE_GROUP], before[PRECOMPUTE_GROUP];
+    for (u32 j0 = 1; j0 < n_tables; j0 += PRECOMPUTE_GROUP) {
+        const u32 g = min(PRECOMPUTE_GROUP, n_tables - j0);
+        Fe<FQ> run = fe_one<FQ>();
+#pragma unroll 1
+        for (u32 t = 0; t < g; t++) {
+#pragma unroll 1
+            for (u32 k = 0; k < shift; k++) p = jac_dbl(p);
+            AffineT<FQ> xy;  // Jacobian x and y wait in the table's slot
+            xy.x = p.x;
+            xy.y = p.y;
+            affine_store(points + ((u64)(j0 + t) * n + i) * C::PW, xy);
+            z[t] = p.z;
+            before[t] = run;
+            run = fe_mul(run, p.z);
+        }
+        Fe<FQ> inv = fe_inv_divsteps<FQ>(run, fe_rcube<FQ>());
+#pragma unroll 1
+        for (u32 t = g; t-- > 0;) {
+            const Fe<FQ> zi = fe_mul(inv, before[t]);
+            inv = fe_mul(inv, z[t]);
+            u32 *slot = points + ((u64)(j0 + t) * n + i) * C::PW;
+            AffineT<FQ> xy = affine_load<FQ>(slot);
+            const Fe<FQ> zi2 = fe_sqr(zi);
+            xy.x = fe_canon(fe_mul(xy.x, zi2));
+            xy.y = fe_canon(fe_mul(xy.y, fe_mul(zi2, zi)));
+            affine_store(slot, xy);
+        }
     }
 }
 
