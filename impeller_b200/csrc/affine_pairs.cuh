@@ -9,6 +9,7 @@
 #pragma once
 
 #include "bn254.cuh"
+#include "launch.cuh"
 
 namespace impeller {
 
@@ -295,6 +296,7 @@ __device__ __forceinline__ Fe<typename C::Fq> pair_y(const u32 *py, u32 e) {
 // back through its pairs.  Blocks take tiles from a counter.
 template <class C, int FROM>
 __global__ void __launch_bounds__(PAIR_BLOCK, PairShape<C>::per_sm) k_affine_pairs(PairArgs a) {
+    grid_wait();
     using FQ = typename C::Fq;
     using S = PairShape<C>;
     extern __shared__ uint4 pair_smem[];
@@ -466,6 +468,7 @@ __host__ __device__ __forceinline__ u32 pair_levels(u64 entries, u64 nb, u64 slo
 // levels' tile counters.
 __global__ void k_pair_plan(const u32 *__restrict__ offsets, u32 nb, u32 slots_min, u32 most, u32 *__restrict__ out,
                             u32 *__restrict__ state) {
+    grid_wait();
     const u32 used = pair_levels(offsets[nb], nb, slots_min, most);
     if (blockIdx.x == 0 && threadIdx.x <= PAIR_MAX_LEVELS) state[threadIdx.x] = threadIdx.x ? 0 : used;
     for (u32 b = blockIdx.x * blockDim.x + threadIdx.x; b <= nb; b += gridDim.x * blockDim.x)

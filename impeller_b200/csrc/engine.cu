@@ -49,20 +49,20 @@ u32 digit_windows(u32 c, u32 curve) {
 #define CURVE_LAUNCH(curve_id, kern, grid, block, smem, st, ...)                      \
     do {                                                                               \
         if ((curve_id) == CURVE_BLS12381)                                              \
-            kern<Bls12381><<<(grid), (block), (smem), (st)>>>(__VA_ARGS__);            \
+            launch_next(kern<Bls12381>, (grid), (block), (smem), (st), __VA_ARGS__);            \
         else                                                                           \
-            kern<Bn254><<<(grid), (block), (smem), (st)>>>(__VA_ARGS__);               \
+            launch_next(kern<Bn254>, (grid), (block), (smem), (st), __VA_ARGS__);               \
     } while (0)
 
 // Launch a digit-recoding kernel for the plan's curve and scalars.
 #define DIGIT_LAUNCH(curve_id, images, kern, grid, block, smem, st, ...)               \
     do {                                                                               \
         if ((curve_id) == CURVE_BLS12381)                                              \
-            kern<Bls12381, false><<<(grid), (block), (smem), (st)>>>(__VA_ARGS__);     \
+            launch_next(kern<Bls12381, false>, (grid), (block), (smem), (st), __VA_ARGS__);     \
         else if (images)                                                               \
-            kern<Bn254, true><<<(grid), (block), (smem), (st)>>>(__VA_ARGS__);         \
+            launch_next(kern<Bn254, true>, (grid), (block), (smem), (st), __VA_ARGS__);         \
         else                                                                           \
-            kern<Bn254, false><<<(grid), (block), (smem), (st)>>>(__VA_ARGS__);        \
+            launch_next(kern<Bn254, false>, (grid), (block), (smem), (st), __VA_ARGS__);        \
     } while (0)
 
 int sm_count(int device) {
@@ -374,7 +374,8 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
         }
         bin_cell[nbins] = (u32)std::min<u64>(cells, 0xffffffffu);
     }
-    p.msd = stiles > 0 && nbins <= SORT_MAX_BINS && cells <= SORT_MAX_CELLS;
+    p.small_sort = p.M == 1 && entries <= SMALL_SORT_ENTRIES && nb <= SMALL_SORT_BUCKETS;
+    p.msd = !p.small_sort && stiles > 0 && nbins <= SORT_MAX_BINS && cells <= SORT_MAX_CELLS;
     if (p.msd) {
         p.nbins = (u32)nbins;
         p.sort_tiles = (u32)stiles;
@@ -410,10 +411,10 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
     };
     lo.o_tables = take(tbytes);
     lo.tables_bytes = tbytes;
-    lo.o_counts = take(p.msd ? 0 : (size_t)p.nb_pad * 4);
-    lo.o_cursor = take(p.msd ? 0 : (size_t)p.nb * 4);
+    lo.o_counts = take(p.msd || p.small_sort ? 0 : (size_t)p.nb_pad * 4);
+    lo.o_cursor = take(p.msd || p.small_sort ? 0 : (size_t)p.nb * 4);
     lo.o_offsets = take((size_t)(p.nb + 1) * 4);
-    lo.o_tiles = take(p.msd ? 0 : (size_t)(p.ntiles + 1) * 4);
+    lo.o_tiles = take(p.msd || p.small_sort ? 0 : (size_t)(p.ntiles + 1) * 4);
     lo.o_entries = take((size_t)std::max<u64>(entries, 1) * 4);
     const size_t ncnt = p.ncells;
     lo.o_cnt = take(p.msd ? (size_t)p.cnt_pad * 4 : 0);
@@ -448,6 +449,7 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
 }
 
 Plan::~Plan() {
+    if (image) cudaFreeAsync(image, nullptr);
     if (staging && staging != ext_staging) cudaFreeHost(staging);
     if (staged) cudaEventDestroy(staged);
     for (auto &set : prof_sets)
@@ -456,7 +458,7 @@ Plan::~Plan() {
 
 // sort (10 kernels two-level, 6 per-entry) + accumulate, 2 fixups, reduce,
 // one per reduction-tree level, final
-u32 Plan::launches() const { return (msd ? 10u : 6u) + (pair_levels ? pair_levels + 2u : 0u) + (phi_points ? 1u : 0u) + 5u + (u32)tree_first.size() - 1u; }
+u32 Plan::launches() const { return (small_sort ? 1u : msd ? 10u : 6u) + (pair_levels ? pair_levels + 2u : 0u) + (phi_points ? 1u : 0u) + 5u + (u32)tree_first.size() - 1u; }
 
 const char *Plan::phase_name(int i) {
     static const char *names[NPHASE] = {"tables", "histogram", "scan", "scatter",
@@ -568,17 +570,17 @@ static cudaError_t launch_pair_levels(int device, u32 curve, u32 levels, PairArg
     CK(cudaFuncSetAttribute(k_affine_pairs<C, FROM_LEVEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     pa.sms = (u32)sm_count(device);
     pa.used = state;
-    k_pair_plan<<<std::max(1u, std::min((pa.nb + 256) / 256, pa.sms * 8)), 256, 0, st>>>(
-        pa.offsets, pa.nb, pair_slots_min((int)pa.sms, curve), levels, offsets, state);
+    launch_next(k_pair_plan, std::max(1u, std::min((pa.nb + 256) / 256, pa.sms * 8)), 256, 0, st, pa.offsets, pa.nb,
+                pair_slots_min((int)pa.sms, curve), levels, offsets, state);
     CK_LAUNCH("k_pair_plan");
     const u32 grid = pa.sms * PairShape<C>::per_sm;
     for (u32 l = 0; l < levels; l++) {
         pa.level = l;
         pa.out = l & 1u ? even : odd;
         pa.next_unit = state + 1 + l;
-        if (l) k_affine_pairs<C, FROM_LEVEL><<<grid, PAIR_BLOCK, smem, st>>>(pa);
-        else if (pa.phi_base != NONE) k_affine_pairs<C, IMAGES><<<grid, PAIR_BLOCK, smem, st>>>(pa);
-        else k_affine_pairs<C, FROM_ENTRIES><<<grid, PAIR_BLOCK, smem, st>>>(pa);
+        if (l) launch_next(k_affine_pairs<C, FROM_LEVEL>, grid, PAIR_BLOCK, smem, st, pa);
+        else if (pa.phi_base != NONE) launch_next(k_affine_pairs<C, IMAGES>, grid, PAIR_BLOCK, smem, st, pa);
+        else launch_next(k_affine_pairs<C, FROM_ENTRIES>, grid, PAIR_BLOCK, smem, st, pa);
         CK_LAUNCH("k_affine_pairs");
         pa.points = pa.out;
     }
@@ -591,14 +593,14 @@ template <int FROM>
 static void launch_accumulate(u32 curve, bool carry, bool images, u32 grid, u32 block, const AccumArgs &aa,
                               cudaStream_t st) {
     if (curve == CURVE_BLS12381) {
-        if (carry) k_accumulate<Bls12381, START_CARRY, FROM><<<grid, block, 0, st>>>(aa);
-        else k_accumulate<Bls12381, ACCUM_START_BLS, FROM><<<grid, block, 0, st>>>(aa);
+        if (carry) launch_next(k_accumulate<Bls12381, START_CARRY, FROM>, grid, block, 0, st, aa);
+        else launch_next(k_accumulate<Bls12381, ACCUM_START_BLS, FROM>, grid, block, 0, st, aa);
     } else if (images) {
-        if (carry) k_accumulate<Bn254, START_CARRY, FROM_IMAGES><<<grid, block, 0, st>>>(aa);
-        else k_accumulate<Bn254, START_CONVERT, FROM_IMAGES><<<grid, block, 0, st>>>(aa);
+        if (carry) launch_next(k_accumulate<Bn254, START_CARRY, FROM_IMAGES>, grid, block, 0, st, aa);
+        else launch_next(k_accumulate<Bn254, START_CONVERT, FROM_IMAGES>, grid, block, 0, st, aa);
     } else {
-        if (carry) k_accumulate<Bn254, START_CARRY, FROM><<<grid, block, 0, st>>>(aa);
-        else k_accumulate<Bn254, START_CONVERT, FROM><<<grid, block, 0, st>>>(aa);
+        if (carry) launch_next(k_accumulate<Bn254, START_CARRY, FROM>, grid, block, 0, st, aa);
+        else launch_next(k_accumulate<Bn254, START_CONVERT, FROM>, grid, block, 0, st, aa);
     }
 }
 
@@ -623,6 +625,7 @@ static cudaError_t sort_smem(int device, u32 curve, int kernel, size_t bytes) {
 
 // Zero n words at p and m words at q.
 __global__ void k_zero_words(u32 *__restrict__ p, u32 n, u32 *__restrict__ q, u32 m) {
+    grid_wait();
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = 0;
     if (blockIdx.x == 0 && threadIdx.x < m) q[threadIdx.x] = 0;
 }
@@ -633,7 +636,7 @@ __global__ void k_zero_words(u32 *__restrict__ p, u32 n, u32 *__restrict__ q, u3
 // when d_image is given, so nothing here queues behind transfers on a copy
 // engine.
 cudaError_t Plan::run_front(void *scratch, const u32 *points, cudaStream_t st, bool record_staged,
-                            const void *d_image, u32 *bucket_out, cudaEvent_t points_ready) {
+                            const void *d_image, u32 *bucket_out, cudaEvent_t points_ready, const u32 *only_scalars) {
     const PlanPtrs p = plan_ptrs(layout, desc_off, win_off, blk_off, tf_off, scratch, nullptr, nullptr, d_image);
     cudaError_t pe;
     MARK(0);
@@ -642,7 +645,15 @@ cudaError_t Plan::run_front(void *scratch, const u32 *points, cudaStream_t st, b
                            cudaMemcpyHostToDevice, st));
         if (record_staged) CK(cudaEventRecord(staged, st));
     }
-    if (msd) {
+    if (small_sort) {
+        MARK(1);
+        MARK(2);
+        MARK(3);
+        DIGIT_LAUNCH(curve, phi_points, k_small_sort, 1, SMALL_SORT_BLOCK, nb * 4, st, p.desc, only_scalars, nb,
+                     p.offsets, p.entries, p.longl);
+        CK_LAUNCH("k_small_sort");
+        MARK(4);
+    } else if (msd) {
         unsigned char *sb = static_cast<unsigned char *>(scratch);
         u32 *cnt = reinterpret_cast<u32 *>(sb + layout.o_cnt);
         u32 *coff = reinterpret_cast<u32 *>(sb + layout.o_coff);
@@ -650,7 +661,7 @@ cudaError_t Plan::run_front(void *scratch, const u32 *points, cudaStream_t st, b
         u32 *ctiles = reinterpret_cast<u32 *>(sb + layout.o_ctiles);
         const u32 ncnt = ncells;
         const unsigned char *img = d_image ? static_cast<const unsigned char *>(d_image) : sb + layout.o_tables;
-        SortArgs sa{p.desc, p.tile_first, reinterpret_cast<const u32 *>(img + bc_off), M, sort_tiles, tile_scalars,
+        SortArgs sa{p.desc, only_scalars, p.tile_first, reinterpret_cast<const u32 *>(img + bc_off), M, sort_tiles, tile_scalars,
                     nbins, nb, segcap, cnt, coff,
                     reinterpret_cast<u32 *>(sb + layout.o_centry),
                     reinterpret_cast<unsigned short *>(sb + layout.o_cfine),
@@ -658,53 +669,53 @@ cudaError_t Plan::run_front(void *scratch, const u32 *points, cudaStream_t st, b
                     reinterpret_cast<u32 *>(sb + layout.o_nsegs), reinterpret_cast<u32 *>(sb + layout.o_seghist),
                     reinterpret_cast<u32 *>(sb + layout.o_segcur), p.offsets, p.entries, p.entries};
         // the scan padding of the tile counts and the long-run counter of the fixups
-        k_zero_words<<<1, 256, 0, st>>>(cnt + ncnt, cnt_pad - ncnt, p.longl, 1);
+        launch_next(k_zero_words, 1, 256, 0, st, cnt + ncnt, cnt_pad - ncnt, p.longl, 1);
         CK_LAUNCH("k_zero_words");
         MARK(1);
         DIGIT_LAUNCH(curve, phi_points, k_coarse_count, sort_tiles, SORT_BLOCK, nbins * 4, st, sa);
         CK_LAUNCH("k_coarse_count");
         MARK(2);
-        k_scan_reduce<<<cscan_tiles, SCAN_BLOCK, 0, st>>>(cnt, ctiles);
+        launch_next(k_scan_reduce, cscan_tiles, SCAN_BLOCK, 0, st, cnt, ctiles);
         CK_LAUNCH("k_scan_reduce");
-        k_scan_tiles<<<1, SCAN_BLOCK, 0, st>>>(ctiles, cscan_tiles);
+        launch_next(k_scan_tiles, 1, SCAN_BLOCK, 0, st, ctiles, cscan_tiles);
         CK_LAUNCH("k_scan_tiles");
-        k_scan_down<<<cscan_tiles, SCAN_BLOCK, 0, st>>>(cnt, ctiles, coff, ccur, ncnt, cscan_tiles);
+        launch_next(k_scan_down, cscan_tiles, SCAN_BLOCK, 0, st, cnt, ctiles, coff, ccur, ncnt, cscan_tiles);
         CK_LAUNCH("k_scan_down");
         MARK(3);
         const size_t scatter_smem = (size_t)2 * nbins * 4 + (size_t)STAGE_ENTRIES * 6;
         CK(sort_smem(device, curve, 0, scatter_smem));
         CURVE_LAUNCH(curve, k_coarse_scatter, sort_tiles, SORT_BLOCK, scatter_smem, st, sa);
         CK_LAUNCH("k_coarse_scatter");
-        k_seg_plan<<<1, FINE_BLOCK, 0, st>>>(sa);
+        launch_next(k_seg_plan, 1, FINE_BLOCK, 0, st, sa);
         CK_LAUNCH("k_seg_plan");
-        k_seg_hist<<<segcap, FINE_BLOCK, 0, st>>>(sa);
+        launch_next(k_seg_hist, segcap, FINE_BLOCK, 0, st, sa);
         CK_LAUNCH("k_seg_hist");
-        k_bin_scan<<<nbins, FINE_BLOCK, 0, st>>>(sa);
+        launch_next(k_bin_scan, nbins, FINE_BLOCK, 0, st, sa);
         CK_LAUNCH("k_bin_scan");
         const size_t seg_smem = (size_t)2 * FINE * 4 + (size_t)SEG_ENTRIES * 6;
         CK(sort_smem(device, curve, 1, seg_smem));
-        k_seg_scatter<<<segcap, FINE_BLOCK, seg_smem, st>>>(sa);
+        launch_next(k_seg_scatter, segcap, FINE_BLOCK, seg_smem, st, sa);
         CK_LAUNCH("k_seg_scatter");
         MARK(4);
     } else {
         // the bucket counts and the long-run counter of the fixups
-        k_zero_words<<<std::max(1u, std::min((nb_pad + 255) / 256, (u32)sm_count(device) * 4)), 256, 0, st>>>(
-            p.counts, nb_pad, p.longl, 1);
+        launch_next(k_zero_words, std::max(1u, std::min((nb_pad + 255) / 256, (u32)sm_count(device) * 4)), 256, 0, st,
+                    p.counts, nb_pad, p.longl, 1);
         CK_LAUNCH("k_zero_words");
         MARK(1);
 
         dim3 hgrid(hist_grid_x, M);
-        DIGIT_LAUNCH(curve, phi_points, k_histogram, hgrid, 256, 0, st, p.desc, p.counts);
+        DIGIT_LAUNCH(curve, phi_points, k_histogram, hgrid, 256, 0, st, p.desc, only_scalars, p.counts);
         CK_LAUNCH("k_histogram");
         MARK(2);
-        k_scan_reduce<<<ntiles, SCAN_BLOCK, 0, st>>>(p.counts, p.tiles);
+        launch_next(k_scan_reduce, ntiles, SCAN_BLOCK, 0, st, p.counts, p.tiles);
         CK_LAUNCH("k_scan_reduce");
-        k_scan_tiles<<<1, SCAN_BLOCK, 0, st>>>(p.tiles, ntiles);
+        launch_next(k_scan_tiles, 1, SCAN_BLOCK, 0, st, p.tiles, ntiles);
         CK_LAUNCH("k_scan_tiles");
-        k_scan_down<<<ntiles, SCAN_BLOCK, 0, st>>>(p.counts, p.tiles, p.offsets, p.cursor, nb, ntiles);
+        launch_next(k_scan_down, ntiles, SCAN_BLOCK, 0, st, p.counts, p.tiles, p.offsets, p.cursor, nb, ntiles);
         CK_LAUNCH("k_scan_down");
         MARK(3);
-        DIGIT_LAUNCH(curve, phi_points, k_scatter, hgrid, 256, 0, st, p.desc, p.cursor, p.entries);
+        DIGIT_LAUNCH(curve, phi_points, k_scatter, hgrid, 256, 0, st, p.desc, only_scalars, p.cursor, p.entries);
         CK_LAUNCH("k_scatter");
         MARK(4);
     }
@@ -714,7 +725,7 @@ cudaError_t Plan::run_front(void *scratch, const u32 *points, cudaStream_t st, b
     u32 *const phi = reinterpret_cast<u32 *>(static_cast<unsigned char *>(scratch) + layout.o_phi);
     const u32 phi_from = phi_points ? phi_base : NONE;
     if (phi_points) {
-        k_images<<<std::min((phi_points + 127) / 128, (u32)sm_count(device) * 16), 128, 0, st>>>(points, phi_points, phi);
+        launch_next(k_images, std::min((phi_points + 127) / 128, (u32)sm_count(device) * 16), 128, 0, st, points, phi_points, phi);
         CK_LAUNCH("k_images");
     }
     const u32 *offsets = p.offsets;
@@ -805,8 +816,8 @@ cudaError_t Plan::launch_chunk(void *scratch, const u32 *points, u32 *acc, bool 
             set_error("bucket accumulators exceed 2^32 words");
             return cudaErrorInvalidValue;
         }
-        k_zero_words<<<std::max(1u, std::min((u32)((words + 255) / 256), (u32)sm_count(device) * 8)), 256, 0, st>>>(
-            acc, (u32)words, nullptr, 0);
+        launch_next(k_zero_words, std::max(1u, std::min((u32)((words + 255) / 256), (u32)sm_count(device) * 8)), 256, 0, st,
+                    acc, (u32)words, nullptr, 0);
         CK_LAUNCH("k_zero_words");
     }
     return run_front(scratch, points, st, true, d_image, acc, points_ready);
@@ -815,6 +826,25 @@ cudaError_t Plan::launch_chunk(void *scratch, const u32 *points, u32 *acc, bool 
 cudaError_t Plan::launch_chunked_tail(void *scratch, const u32 *acc, u32 *results, int carry_mode, cudaStream_t st,
                                       u32 *carry_ext, const void *d_image) {
     return run_tail(scratch, acc, true, results, carry_mode, st, carry_ext, d_image);
+}
+
+cudaError_t Plan::run_one(void *scratch, const u32 *points, const u32 *scalars, u32 *results, cudaStream_t st) {
+    if (!image) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(st, &cap));
+        // memory allocated in a capture would belong to its graph
+        if (cap != cudaStreamCaptureStatusNone) return enqueue(scratch, points, &scalars, results, 0, st);
+        cudaError_t e = scratch_alloc(&image, tables.size(), device, st);
+        if (e != cudaSuccess) {
+            image = nullptr;
+            return e;
+        }
+        CK(cudaMemcpyAsync(image, tables.data(), tables.size(), cudaMemcpyHostToDevice, st));
+    }
+    cudaError_t e = run_front(scratch, points, st, false, image, nullptr, nullptr, scalars);
+    if (e != cudaSuccess) return e;
+    const u32 *buckets = reinterpret_cast<const u32 *>(static_cast<unsigned char *>(scratch) + layout.o_buckets);
+    return run_tail(scratch, buckets, false, results, 0, st, nullptr, image);
 }
 
 cudaError_t Plan::enqueue(void *scratch, const u32 *points, const u32 *const *scalars, u32 *results, int carry_mode,
@@ -1137,12 +1167,12 @@ cudaError_t impeller_ctx_destroy(impeller_ctx *ctx) {
     cudaDeviceSynchronize();
     if (ctx->owns) cudaFree(const_cast<u32 *>(ctx->points));
     if (ctx->tables) cudaFree(ctx->tables);
+    ctx->plans.clear();  // they hold images in the scratch pool
     if (ctx->scratch) cudaFreeAsync(ctx->scratch, nullptr);
     if (ctx->held) scratch_release(ctx->device);
     if (ctx->d_scalars) cudaFree(ctx->d_scalars);
     if (ctx->d_result) cudaFree(ctx->d_result);
     if (ctx->done) cudaEventDestroy(ctx->done);
-    ctx->plans.clear();
     delete ctx;
     return cudaSuccess;
 }
@@ -1212,8 +1242,7 @@ static cudaError_t ctx_run_locked(impeller_ctx *ctx, const uint32_t *d_scalars, 
     }
     if (e != cudaSuccess) return e;
     CK(cudaStreamWaitEvent(stream, ctx->done, 0));
-    const u32 *sc[1] = {d_scalars};
-    e = p->enqueue(ctx->scratch, ctx_point_base(ctx), sc, d_result, 0, stream);
+    e = p->run_one(ctx->scratch, ctx_point_base(ctx), d_scalars, d_result, stream);
     if (e != cudaSuccess) return e;
     CK(cudaEventRecord(ctx->done, stream));
     return cudaSuccess;

@@ -127,6 +127,12 @@ class Plan {
     size_t image_bytes() const;
     void write_image(void *dst, const u32 *const *scalars) const;
 
+    // One MSM (M == 1) whose table image stays on the device between runs: no
+    // copy and no host buffer per run; the scalars come as a kernel argument.
+    // Runs on different streams have to be ordered by the caller; the device's
+    // scratch pool must be held.
+    cudaError_t run_one(void *scratch, const u32 *points, const u32 *scalars, u32 *results, cudaStream_t stream);
+
     size_t scratch_bytes() const { return layout.bytes; }
     u32 launches() const;
     u32 *carry_ptr(void *scratch) const;
@@ -144,6 +150,7 @@ class Plan {
     u32 hist_grid_x = 1;
     // two-level sort (msd) or per-entry atomic bucket sort
     bool msd = false;
+    bool small_sort = false;  // k_small_sort instead of either
     u32 nbins = 0, sort_tiles = 0, tile_scalars = 0, segcap = 0, cnt_pad = 0, cscan_tiles = 0, ncells = 0;
     std::vector<MsmShape> shapes;
     PlanLayout layout{};
@@ -163,10 +170,12 @@ class Plan {
     // bucket_out: accumulate into these buckets, each starting from its
     // current value (streamed chunks); null = the plan's own buckets, fresh.
     cudaError_t run_front(void *scratch, const u32 *points, cudaStream_t stream, bool record_staged,
-                          const void *d_image, u32 *bucket_out = nullptr, cudaEvent_t points_ready = nullptr);
+                          const void *d_image, u32 *bucket_out = nullptr, cudaEvent_t points_ready = nullptr,
+                          const u32 *only_scalars = nullptr);
     cudaError_t run_tail(void *scratch, const u32 *buckets, bool dense, u32 *results, int carry_mode,
                          cudaStream_t stream, u32 *carry_ext, const void *d_image);
 
+    void *image = nullptr;       // device copy of the tables (run_one)
     void *staging = nullptr;     // pinned copy of the tables
     void *ext_staging = nullptr; // caller-owned staging (set_staging)
     size_t ext_cap = 0;

@@ -1,0 +1,35 @@
+// Kernel launches that follow one another closely.
+//
+// A chain of kernels of a few microseconds each pays for every hand-over: the
+// next kernel is only set up once the previous one has drained.  launch_next
+// lets it be set up beside the previous kernel (programmatic stream
+// serialization); grid_wait, the first thing such a kernel does, waits until
+// the previous kernel has completed and its writes are visible, so that the
+// order of all memory accesses is as before.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace impeller {
+
+__device__ __forceinline__ void grid_wait() {
+    asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// kern<<<grid, block, smem, st>>>(args...) for a kernel that starts with grid_wait.
+template <class... P, class... A>
+inline cudaError_t launch_next(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
+}  // namespace impeller

@@ -31,6 +31,7 @@
 #include "affine_pairs.cuh"
 #include "bn254.cuh"
 #include "glv.cuh"
+#include "launch.cuh"
 
 namespace impeller {
 
@@ -151,15 +152,17 @@ __device__ __forceinline__ void for_each_digit(const MsmDesc &d, const Fe<typena
 // Every lane of the warp runs the same number of windows, so the match is
 // always taken with the full warp present.
 template <class C, bool GLV>
-__global__ void k_histogram(const MsmDesc *__restrict__ descs, u32 *__restrict__ counts) {
+__global__ void k_histogram(const MsmDesc *__restrict__ descs, const u32 *only_scalars, u32 *__restrict__ counts) {
+    grid_wait();
     const MsmDesc d = descs[blockIdx.y];
+    const u32 *const scalars = only_scalars ? only_scalars : d.scalars;
     const u32 B = 1u << (d.c - 1);
     const u32 lane = threadIdx.x & 31u;
     const u32 stride = gridDim.x * blockDim.x;
     for (u32 base = blockIdx.x * blockDim.x; base < d.n; base += stride) {
         const u32 i = base + threadIdx.x;
         const bool live = i < d.n;
-        const Fe<typename C::Fr> v = live ? fe_from_mont<typename C::Fr>(fe_load<typename C::Fr>(d.scalars + 8ull * i))
+        const Fe<typename C::Fr> v = live ? fe_from_mont<typename C::Fr>(fe_load<typename C::Fr>(scalars + 8ull * i))
                                           : fe_zero<typename C::Fr>();
         for_each_digit<C, GLV>(d, v, [&](u32 pw, u32, u32 mag, u32) {
             const u32 key = mag ? d.bucket_base + pw * B + mag - 1 : NONE;
@@ -170,15 +173,17 @@ __global__ void k_histogram(const MsmDesc *__restrict__ descs, u32 *__restrict__
 }
 
 template <class C, bool GLV>
-__global__ void k_scatter(const MsmDesc *__restrict__ descs, u32 *__restrict__ cursor, u32 *__restrict__ entries) {
+__global__ void k_scatter(const MsmDesc *__restrict__ descs, const u32 *only_scalars, u32 *__restrict__ cursor, u32 *__restrict__ entries) {
+    grid_wait();
     const MsmDesc d = descs[blockIdx.y];
+    const u32 *const scalars = only_scalars ? only_scalars : d.scalars;
     const u32 B = 1u << (d.c - 1);
     const u32 lane = threadIdx.x & 31u;
     const u32 stride = gridDim.x * blockDim.x;
     for (u32 base = blockIdx.x * blockDim.x; base < d.n; base += stride) {
         const u32 i = base + threadIdx.x;
         const bool live = i < d.n;
-        const Fe<typename C::Fr> v = live ? fe_from_mont<typename C::Fr>(fe_load<typename C::Fr>(d.scalars + 8ull * i))
+        const Fe<typename C::Fr> v = live ? fe_from_mont<typename C::Fr>(fe_load<typename C::Fr>(scalars + 8ull * i))
                                           : fe_zero<typename C::Fr>();
         for_each_digit<C, GLV>(d, v, [&](u32 pw, u32 table, u32 mag, u32 sign) {
             const u32 key = mag ? d.bucket_base + pw * B + mag - 1 : NONE;
@@ -193,6 +198,58 @@ __global__ void k_scatter(const MsmDesc *__restrict__ descs, u32 *__restrict__ c
             }
         });
     }
+}
+
+// The whole sort of one small MSM in one block: count the digits per bucket in
+// shared memory, scan, place.  The digits are recoded twice; at these sizes
+// the ten launches of the two-level sort are what costs (n = 1000, 32 digits:
+// 0.085 ms with them).
+static constexpr u32 SMALL_SORT_BLOCK = 1024;
+static constexpr u32 SMALL_SORT_ENTRIES = 96 * 1024;  // digits
+static constexpr u32 SMALL_SORT_BUCKETS = 8192;       // 32 KB of shared memory
+
+__device__ __forceinline__ u32 block_scan_excl(u32 v, u32 &total, u32 *warp_tot);
+
+template <class C, bool GLV>
+__global__ void __launch_bounds__(SMALL_SORT_BLOCK)
+k_small_sort(const MsmDesc *__restrict__ descs, const u32 *only_scalars, u32 nb, u32 *__restrict__ offsets,
+             u32 *__restrict__ entries, u32 *__restrict__ long_list) {
+    grid_wait();
+    extern __shared__ u32 cur[];  // nb
+    __shared__ u32 warp_tot[32];
+    const MsmDesc d = descs[0];
+    const u32 *const scalars = only_scalars ? only_scalars : d.scalars;
+    const u32 B = 1u << (d.c - 1), t = threadIdx.x;
+    for (u32 b = t; b < nb; b += SMALL_SORT_BLOCK) cur[b] = 0;
+    if (t == 0) long_list[0] = 0;
+    __syncthreads();
+    auto digits = [&](auto &&emit) {
+        for (u32 i = t; i < d.n; i += SMALL_SORT_BLOCK) {
+            const Fe<typename C::Fr> v = fe_from_mont<typename C::Fr>(fe_load<typename C::Fr>(scalars + 8ull * i));
+            for_each_digit<C, GLV>(d, v, [&](u32 pw, u32 table, u32 mag, u32 sign) {
+                if (mag) emit(d.bucket_base + pw * B + mag - 1, ((d.table_base + table * d.table_stride + i) << 1) | sign);
+            });
+        }
+    };
+    digits([&](u32 key, u32) { atomicAdd(&cur[key], 1u); });
+    __syncthreads();
+    const u32 per = (nb + SMALL_SORT_BLOCK - 1) / SMALL_SORT_BLOCK, b0 = t * per;
+    u32 sum = 0;
+    for (u32 k = 0; k < per; k++)
+        if (b0 + k < nb) sum += cur[b0 + k];
+    u32 total;
+    u32 run = block_scan_excl(sum, total, warp_tot);
+    for (u32 k = 0; k < per; k++) {
+        if (b0 + k < nb) {
+            const u32 m = cur[b0 + k];
+            cur[b0 + k] = run;
+            offsets[b0 + k] = run;
+            run += m;
+        }
+    }
+    if (t == 0) offsets[nb] = total;
+    __syncthreads();
+    digits([&](u32 key, u32 e) { entries[atomicAdd(&cur[key], 1u)] = e; });
 }
 
 // ------------------------------------------------- two-level counting sort
@@ -233,6 +290,7 @@ static_assert(FINE == FINE_BLOCK, "k_seg_scatter gives every bucket of a bin one
 
 struct SortArgs {
     const MsmDesc *descs;
+    const u32 *only_scalars;  // not null: the scalars of the plan's one MSM
     const u32 *tile_first;  // M + 1: first sort tile of each MSM
     const u32 *bin_cell;    // nbins + 1: first count cell of each bin; [nbins] = cells
     u32 M, ntiles, tile_scalars, nbins, nb, segcap;
@@ -295,10 +353,12 @@ __device__ __forceinline__ void sort_tile(const SortArgs &a, u32 tile, u32 &m, u
 
 template <class C, bool GLV>
 __global__ void __launch_bounds__(SORT_BLOCK) k_coarse_count(SortArgs a) {
+    grid_wait();
     extern __shared__ u32 hist[];  // nbins
     u32 m, start, end;
     sort_tile(a, blockIdx.x, m, start, end);
     const MsmDesc d = a.descs[m];
+    const u32 *const scalars = a.only_scalars ? a.only_scalars : d.scalars;
     const u32 B = 1u << (d.c - 1);
     // this MSM's bins
     const u32 blo = d.bucket_base >> FINE_BITS, bhi = (d.bucket_base + d.n_windows * B - 1u) >> FINE_BITS;
@@ -310,7 +370,7 @@ __global__ void __launch_bounds__(SORT_BLOCK) k_coarse_count(SortArgs a) {
     for (u32 base = start; base < end; base += blockDim.x) {
         const u32 i = base + threadIdx.x;
         const bool live = i < end;
-        const Fe<typename C::Fr> v = live ? fe_from_mont<typename C::Fr>(fe_load<typename C::Fr>(d.scalars + 8ull * i))
+        const Fe<typename C::Fr> v = live ? fe_from_mont<typename C::Fr>(fe_load<typename C::Fr>(scalars + 8ull * i))
                                           : fe_zero<typename C::Fr>();
         u32 *kw = kp + (i - start);
         for_each_digit<C, GLV>(d, v, [&](u32 pw, u32, u32 mag, u32 sign) {
@@ -337,6 +397,7 @@ __global__ void __launch_bounds__(SORT_BLOCK) k_coarse_count(SortArgs a) {
 // own other bins.
 template <class C>
 __global__ void __launch_bounds__(SORT_BLOCK, 2) k_coarse_scatter(SortArgs a) {
+    grid_wait();
     extern __shared__ u32 sm[];
     __shared__ u32 warp_tot[32];
     u32 *delta = sm, *cur = sm + a.nbins, *stage_e = sm + 2 * a.nbins;
@@ -411,6 +472,7 @@ __global__ void __launch_bounds__(SORT_BLOCK, 2) k_coarse_scatter(SortArgs a) {
 
 // One block: every bin's segments (at most SEG_ENTRIES entries each).
 __global__ void __launch_bounds__(FINE_BLOCK) k_seg_plan(SortArgs a) {
+    grid_wait();
     __shared__ u32 warp_tot[32];
     const u32 per = (a.nbins + blockDim.x - 1) / blockDim.x;
     const u32 b0 = threadIdx.x * per;
@@ -452,6 +514,7 @@ __device__ __forceinline__ void hist8(u32 *hist, uint4 q) {
 }
 
 __global__ void __launch_bounds__(FINE_BLOCK) k_seg_hist(SortArgs a) {
+    grid_wait();
     __shared__ u32 hist[FINE];
     if (blockIdx.x >= a.nsegs[0]) return;
     const uint4 sg = a.segs[blockIdx.x];
@@ -482,6 +545,7 @@ __global__ void __launch_bounds__(FINE_BLOCK) k_seg_hist(SortArgs a) {
 // segments (their cursors) and the bucket's total; then a scan over the
 // bin's buckets gives the bucket offsets.
 __global__ void __launch_bounds__(FINE_BLOCK) k_bin_scan(SortArgs a) {
+    grid_wait();
     __shared__ u32 warp_tot[32];
     const u32 b = blockIdx.x;
     const uint2 bs = a.bin_seg[b];
@@ -523,6 +587,7 @@ __device__ __forceinline__ void place4(u32 *lcur, u32 *stage_e, unsigned short *
 }
 
 __global__ void __launch_bounds__(FINE_BLOCK) k_seg_scatter(SortArgs a) {
+    grid_wait();
     extern __shared__ u32 sm[];
     __shared__ u32 warp_tot[32];
     if (blockIdx.x >= a.nsegs[0]) return;
@@ -588,6 +653,7 @@ __device__ __forceinline__ u32 block_exclusive_scan(u32 v, u32 &total) {
 
 // counts must be padded to a multiple of SCAN_TILE with zeros.
 __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_reduce(const u32 *__restrict__ counts, u32 *__restrict__ tile_sums) {
+    grid_wait();
     const uint4 *p = reinterpret_cast<const uint4 *>(counts + (size_t)blockIdx.x * SCAN_TILE) + threadIdx.x * 4;
     u32 s = 0;
 #pragma unroll
@@ -603,6 +669,7 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_reduce(const u32 *__restric
 // Single block: exclusive scan of the tile sums in place; tile_sums[ntiles]
 // receives the grand total.
 __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_tiles(u32 *__restrict__ tile_sums, u32 ntiles) {
+    grid_wait();
     u32 carry = 0;
     for (u32 base = 0; base < ntiles; base += SCAN_BLOCK) {
         u32 i = base + threadIdx.x;
@@ -618,6 +685,7 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_tiles(u32 *__restrict__ til
 __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_down(const u32 *__restrict__ counts, const u32 *__restrict__ tile_sums,
                                                    u32 *__restrict__ offsets, u32 *__restrict__ cursor, u32 nb,
                                                    u32 ntiles) {
+    grid_wait();
     const size_t base = (size_t)blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_PER_THREAD;
     const uint4 *p = reinterpret_cast<const uint4 *>(counts + base);
     u32 v[SCAN_PER_THREAD];
@@ -683,6 +751,7 @@ __device__ __forceinline__ AffineT<typename C::Fq> load_entry_point(const u32 *_
 
 // x of the points' images under the endomorphism: beta x.
 __global__ void k_images(const u32 *__restrict__ points, u32 n, u32 *__restrict__ phi) {
+    grid_wait();
     const Fq beta = {GLV_BETA};
     for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         fe_store(phi + 8ull * i, fe_mul<FqP>(fe_load<FqP>(points + 16ull * i), beta));
@@ -738,6 +807,7 @@ enum : int { START_CONVERT = 0, START_IDENTITY = 1, START_CARRY = 2 };
 // kernel that picked at run time was 4 % slower on BN254.
 template <class C, int START = START_CONVERT, int FROM = FROM_ENTRIES>
 __global__ void __launch_bounds__(AccumShape<C>::threads, AccumShape<C>::per_sm) k_accumulate(AccumArgs a) {
+    grid_wait();
     using FQ = typename C::Fq;
     const u32 levels = a.pair_state ? *a.pair_state : 0;
     if ((FROM == FROM_LEVEL) != (levels != 0)) return;
@@ -840,6 +910,7 @@ struct FixupArgs {
 // The bucket continues as the first piece (record 2t') of slices t+1 .. t1.
 template <class C>
 __global__ void k_fixup_short(FixupArgs f) {
+    grid_wait();
     using FQ = typename C::Fq;
     const u32 t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= f.T) return;
@@ -868,6 +939,7 @@ __global__ void k_fixup_short(FixupArgs f) {
 static constexpr u32 WIDE_BLOCK = 128;
 template <class C>
 __global__ void k_fixup_long(FixupArgs f, u32 wide_blocks) {
+    grid_wait();
     using FQ = typename C::Fq;
     __shared__ __align__(16) u32 part[WIDE_BLOCK / 32][C::XW];
     const u32 lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
@@ -982,6 +1054,7 @@ __device__ __forceinline__ u32 ilog2(u32 x) { return 31 - __clz(x); }
 // registers (254 instead of 168: spills 2 KB -> 80 B, 4 % faster).
 template <class C>
 __global__ void __launch_bounds__(REDUCE_BLOCK, C::XW == 32 ? REDUCE_BLOCKS_PER_SM : 2) k_reduce(ReduceArgs r) {
+    grid_wait();
     using FQ = typename C::Fq;
     using Xz = XyzzT<FQ>;
     const uint2 blk = r.blocks[blockIdx.x];
@@ -1140,6 +1213,7 @@ struct TreeArgs {
 
 template <class C>
 __global__ void __launch_bounds__(TREE_BLOCK, C::XW == 32 ? 2 : 1) k_reduce_tree(TreeArgs a) {
+    grid_wait();
     using FQ = typename C::Fq;
     using Xz = XyzzT<FQ>;
     const u32 g = blockIdx.x * TREE_WARPS + (threadIdx.x >> 5);
@@ -1201,6 +1275,7 @@ struct FinalArgs {
 // then the carry and the affine form.
 template <class C>
 __global__ void k_final(FinalArgs f) {
+    grid_wait();
     using FQ = typename C::Fq;
     const u32 m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= f.M) return;

@@ -203,7 +203,7 @@ extern "C" cudaError_t impeller_msm_device_noalloc(const uint32_t *d_points, con
     NA_LAUNCHED("k_noalloc_tables");
     NA_CK(cudaMemsetAsync(counts, 0, (size_t)NB_PAD * 4, stream));
     const dim3 hgrid((u32)((n + 255) / 256), 1);
-    K::k_histogram<K::Bn254, false><<<hgrid, 256, 0, stream>>>(desc, counts);
+    K::k_histogram<K::Bn254, false><<<hgrid, 256, 0, stream>>>(desc, nullptr, counts);
     NA_LAUNCHED("k_histogram");
     K::k_scan_reduce<<<NTILES, K::SCAN_BLOCK, 0, stream>>>(counts, tiles);
     NA_LAUNCHED("k_scan_reduce");
@@ -211,7 +211,7 @@ extern "C" cudaError_t impeller_msm_device_noalloc(const uint32_t *d_points, con
     NA_LAUNCHED("k_scan_tiles");
     K::k_scan_down<<<NTILES, K::SCAN_BLOCK, 0, stream>>>(counts, tiles, offsets, cursor, NB, NTILES);
     NA_LAUNCHED("k_scan_down");
-    K::k_scatter<K::Bn254, false><<<hgrid, 256, 0, stream>>>(desc, cursor, entries);
+    K::k_scatter<K::Bn254, false><<<hgrid, 256, 0, stream>>>(desc, nullptr, cursor, entries);
     NA_LAUNCHED("k_scatter");
     AccumArgs aa{entries, offsets, NB, d_points, buckets, recb, recp};
     K::k_accumulate<K::Bn254><<<ACC_BLOCKS, ACC_THREADS, 0, stream>>>(aa);

@@ -33,6 +33,7 @@
 #include "../../include/impeller_ntt.h"
 #include "bn254.cuh"
 #include "engine.h"
+#include "launch.cuh"
 
 using namespace ec;
 
@@ -116,6 +117,7 @@ __device__ __forceinline__ Fe<F> twiddle(const u32 *tw, u32 e) {
 template <class F, bool RECOMP>
 __global__ void __launch_bounds__(THREADS, 3)
 k_ntt_pass(View v, const u32 *tw, u32 L, u32 lo, u32 R, u32 logC, int rev_out) {
+    impeller::grid_wait();
     extern __shared__ uint4 ntt_smem[];
     const u32 tile_log = R + logC;
     const u32 tsize = 1u << tile_log;
@@ -241,6 +243,7 @@ k_ntt_pass(View v, const u32 *tw, u32 L, u32 lo, u32 R, u32 logC, int rev_out) {
 // consecutive elements each) and writes each into the other's place.
 template <class F>
 __global__ void __launch_bounds__(256) k_ntt_reverse(View v, u32 L) {
+    impeller::grid_wait();
     __shared__ uint4 tl[2][16 * 17 * 2];  // 16 x 16 elements, rows padded to 17
     const u32 m = L - 2 * REV_T;
     const u32 b = blockIdx.x;
@@ -281,6 +284,7 @@ __global__ void k_omegas(const u32 *unit, u32 *omegas, u32 count) {
 // entries from 3 TAB on are the fourth table's, shifted by L - 11.
 template <class F>
 __global__ void k_pow_tables(const u32 *omegas, u32 *tab, u32 n_omegas, u32 count, u32 L) {
+    impeller::grid_wait();
     const u32 g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= count) return;
     const u32 t = g / TAB, j = g % TAB, first = t < 3 ? TAB_LOG * t : L - TAB_LOG;
@@ -302,6 +306,7 @@ __global__ void k_powers(const u32 *tab, u32 *out, u64 len, u64 step) {
 // poly[i] *= powers[((begin + i) mod plen) mod pnum]
 template <class F>
 __global__ void k_distribute_powers(View v, u64 len, const u32 *powers, u64 pnum, u64 begin, u64 plen) {
+    impeller::grid_wait();
     const bool direct = begin == 0 && plen >= len && pnum >= len;
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (u64)gridDim.x * blockDim.x) {
         const u64 k = direct ? i : ((begin + i) % plen) % pnum;
@@ -394,11 +399,12 @@ cudaError_t run_ntt(const View &v, const u32 *tw, u32 L, cudaStream_t st) {
     for (const PassPlan &pp : passes) {
         const u32 tile_log = pp.R + pp.logC;
         const u64 grid = 1ull << (L - tile_log);
-        kern<<<(unsigned)grid, THREADS, (size_t)32 << tile_log, st>>>(v, tw, L, pp.lo, pp.R, pp.logC, single ? 1 : 0);
+        impeller::launch_next(kern, (unsigned)grid, THREADS, (size_t)32 << tile_log, st, v, tw, L, pp.lo, pp.R, pp.logC,
+                              single ? 1 : 0);
         NTT_CK(launched("k_ntt_pass"));
     }
     if (!single) {
-        k_ntt_reverse<F><<<1u << (L - 2 * REV_T), 256, 0, st>>>(v, L);
+        impeller::launch_next(k_ntt_reverse<F>, 1u << (L - 2 * REV_T), 256, 0, st, v, L);
         NTT_CK(launched("k_ntt_reverse"));
     }
     return cudaSuccess;
@@ -409,7 +415,7 @@ cudaError_t run_ntt(const View &v, const u32 *tw, u32 L, cudaStream_t st) {
 template <class F>
 cudaError_t pow_tables(const u32 *d_omegas, u32 n_om, u32 *d_tab, cudaStream_t st, u32 L = 0) {
     const u32 count = 3 * TAB + (L > TILE_LOG ? TAB / 2 : 0);
-    k_pow_tables<F><<<(count + 255) / 256, 256, 0, st>>>(d_omegas, d_tab, n_om, count, L);
+    impeller::launch_next(k_pow_tables<F>, (count + 255) / 256, 256, 0, st, d_omegas, d_tab, n_om, count, L);
     return launched("k_pow_tables");
 }
 
@@ -555,8 +561,8 @@ cudaError_t distribute_impl(PolyPtr poly, const u32 *powers, u64 pnum, cudaStrea
         plen = ps->len;
     }
     const u64 blocks = (poly.len + 255) / 256;
-    k_distribute_powers<F><<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, st>>>(v, poly.len, powers,
-                                                                                          pnum, begin, plen);
+    impeller::launch_next(k_distribute_powers<F>, (unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, st, v,
+                          poly.len, powers, pnum, begin, plen);
     return launched("k_distribute_powers");
 }
 
