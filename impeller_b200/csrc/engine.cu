@@ -54,6 +54,15 @@ u32 digit_windows(u32 c, u32 curve) {
             launch_next(kern<Bn254>, (grid), (block), (smem), (st), __VA_ARGS__);               \
     } while (0)
 
+// The same after the previous kernel has drained.
+#define CURVE_LAUNCH_PLAIN(curve_id, kern, grid, block, smem, st, ...)                 \
+    do {                                                                               \
+        if ((curve_id) == CURVE_BLS12381)                                              \
+            kern<Bls12381><<<(grid), (block), (smem), (st)>>>(__VA_ARGS__);            \
+        else                                                                           \
+            kern<Bn254><<<(grid), (block), (smem), (st)>>>(__VA_ARGS__);               \
+    } while (0)
+
 // Launch a digit-recoding kernel for the plan's curve and scalars.
 #define DIGIT_LAUNCH(curve_id, images, kern, grid, block, smem, st, ...)               \
     do {                                                                               \
@@ -185,7 +194,7 @@ static u32 pair_level_count(u64 entries, u64 nb, int sms, u32 curve) {
     return pair_levels(entries, nb, pair_slots_min(sms, curve), PAIR_MAX_LEVELS);
 }
 
-bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool pairs) {
+bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool resident, bool no_pairs) {
     p.device = device;
     p.shapes = shapes;
     p.M = (u32)shapes.size();
@@ -277,7 +286,11 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
     // two that keeps the lanes at most REDUCE_LANES_PER_SM per SM: beyond
     // that the lanes compete for issue slots and the chain length no longer
     // sets the time.
-    const u64 target = (u64)sms * REDUCE_LANES_PER_SM;
+    // Up to REDUCE_PAIRS_MAX buckets two lanes share a chunk (half the time per
+    // addition, half the additions at once): L leaves each warp a scheduler of
+    // its own.
+    p.reduce_pairs = nb <= REDUCE_PAIRS_MAX;
+    const u64 target = p.reduce_pairs ? (u64)sms * 64 : (u64)sms * REDUCE_LANES_PER_SM;
     u32 L = 1;
     while (nb / L > target && L < (1u << 30)) L <<= 1;
     std::vector<uint2> rblocks;
@@ -285,7 +298,7 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
     for (u32 wi = 0; wi < wins.size(); wi++) {
         WinDesc &w = wins[wi];
         w.chunk = std::min(L, w.nbuckets);
-        const u32 nthreads = (w.nbuckets + w.chunk - 1) / w.chunk;
+        const u32 nthreads = (w.nbuckets + w.chunk - 1) / w.chunk * (p.reduce_pairs ? 2 : 1);
         const u32 nblocks = (nthreads + REDUCE_BLOCK - 1) / REDUCE_BLOCK;
         w.part_base = nparts;
         w.nparts = nblocks * REDUCE_WARPS;  // one partial per reduce warp
@@ -303,7 +316,7 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
         for (u32 wi = 0; wi < nw; wi++) {
             base[wi] = wins[wi].part_base;
             count[wi] = wins[wi].nparts;
-            shift[wi] = 31 - __builtin_clz(wins[wi].chunk) + 5;
+            shift[wi] = 31 - __builtin_clz(wins[wi].chunk) + (p.reduce_pairs ? 4 : 5);
         }
         u32 left = nw;
         while (left) {
@@ -331,7 +344,7 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
     p.nrblocks = (u32)rblocks.size();
 
     const bool bls = p.curve == CURVE_BLS12381;
-    p.pair_levels = pairs ? pair_level_count(entries, nb, sms, p.curve) : 0;
+    p.pair_levels = resident && !no_pairs ? pair_level_count(entries, nb, sms, p.curve) : 0;
 
     // accumulate: persistent threads (every resident slot), at least 8 entries each
     const u32 accum_threads = bls ? AccumShape<Bls12381>::threads : AccumShape<Bn254>::threads;
@@ -340,6 +353,12 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
     p.accum_blocks =
         (u32)std::max<u64>(1, std::min<u64>(full_blocks, (want_threads + accum_threads - 1) / accum_threads));
     p.accum_block = accum_threads;
+    if (resident && p.accum_blocks < full_blocks) {
+        // few threads: the same number in smaller blocks, over every SM
+        const u64 per_sm = (want_threads + sms - 1) / sms;
+        p.accum_block = std::min(accum_threads, (u32)std::max<u64>(32, align_up(per_sm, 32)));
+        p.accum_blocks = (u32)std::max<u64>(1, (want_threads + p.accum_block - 1) / p.accum_block);
+    }
     const u32 T = p.accum_blocks * p.accum_block;
     p.long_cap = T;
     p.hist_grid_x = (u32)std::max<u64>(1, std::min<u64>((u64)sms * 8, (nmax + 255) / 256));
@@ -374,7 +393,7 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
         }
         bin_cell[nbins] = (u32)std::min<u64>(cells, 0xffffffffu);
     }
-    p.small_sort = p.M == 1 && entries <= SMALL_SORT_ENTRIES && nb <= SMALL_SORT_BUCKETS;
+    p.small_sort = resident && p.M == 1 && entries <= SMALL_SORT_ENTRIES && nb <= SMALL_SORT_BUCKETS;
     p.msd = !p.small_sort && stiles > 0 && nbins <= SORT_MAX_BINS && cells <= SORT_MAX_CELLS;
     if (p.msd) {
         p.nbins = (u32)nbins;
@@ -441,7 +460,8 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
     lo.o_parts = take((size_t)nparts * XB);
     lo.o_parts_s = take((size_t)nparts * XB);
     lo.o_wres = take((size_t)wins.size() * XB);
-    lo.o_long = take((size_t)(1 + p.long_cap) * 4);
+    // counts of wide and long runs, the long runs, the wide ones
+    lo.o_long = take((size_t)(2 + p.long_cap + T / FIXUP_WARP_MAX + 1) * 4);
     lo.o_carry = take((size_t)p.M * XB);
     lo.o_results = take((size_t)p.M * PB);
     lo.bytes = off;
@@ -669,7 +689,7 @@ cudaError_t Plan::run_front(void *scratch, const u32 *points, cudaStream_t st, b
                     reinterpret_cast<u32 *>(sb + layout.o_nsegs), reinterpret_cast<u32 *>(sb + layout.o_seghist),
                     reinterpret_cast<u32 *>(sb + layout.o_segcur), p.offsets, p.entries, p.entries};
         // the scan padding of the tile counts and the long-run counter of the fixups
-        launch_next(k_zero_words, 1, 256, 0, st, cnt + ncnt, cnt_pad - ncnt, p.longl, 1);
+        launch_next(k_zero_words, 1, 256, 0, st, cnt + ncnt, cnt_pad - ncnt, p.longl, 2);
         CK_LAUNCH("k_zero_words");
         MARK(1);
         DIGIT_LAUNCH(curve, phi_points, k_coarse_count, sort_tiles, SORT_BLOCK, nbins * 4, st, sa);
@@ -700,7 +720,7 @@ cudaError_t Plan::run_front(void *scratch, const u32 *points, cudaStream_t st, b
     } else {
         // the bucket counts and the long-run counter of the fixups
         launch_next(k_zero_words, std::max(1u, std::min((nb_pad + 255) / 256, (u32)sm_count(device) * 4)), 256, 0, st,
-                    p.counts, nb_pad, p.longl, 1);
+                    p.counts, nb_pad, p.longl, 2);
         CK_LAUNCH("k_zero_words");
         MARK(1);
 
@@ -753,7 +773,8 @@ cudaError_t Plan::run_front(void *scratch, const u32 *points, cudaStream_t st, b
     MARK(5);
 
     const u32 T = accum_blocks * accum_block;
-    FixupArgs fa{offsets, nb, T, p.recb, p.recp, buckets, p.longl, long_cap, FIXUP_WARP_MAX};
+    FixupArgs fa{offsets, nb, T, p.recb, p.recp, buckets, p.longl + 1, long_cap, FIXUP_WARP_MAX, p.longl,
+                 p.longl + 2 + long_cap};
     CURVE_LAUNCH(curve, k_fixup_short, (T + 255) / 256, 256, 0, st, fa);
     CK_LAUNCH("k_fixup_short");
     const u32 wide_blocks = (u32)sm_count(device);
@@ -770,7 +791,10 @@ cudaError_t Plan::run_tail(void *scratch, const u32 *buckets, bool dense, u32 *r
     const PlanPtrs p = plan_ptrs(layout, desc_off, win_off, blk_off, tf_off, scratch, carry_ext, results, d_image);
     cudaError_t pe;
     ReduceArgs ra{p.wins, p.blk, pair_levels ? p.level_offsets : p.offsets, buckets, p.parts, p.parts_s, dense ? 1u : 0u};
-    CURVE_LAUNCH(curve, k_reduce, nrblocks, REDUCE_BLOCK, 0, st, ra);
+    // k_reduce's blocks fill half of the chip: set up ahead they crowd onto the
+    // SMs that the fixups leave first (2^20 skewed: 1.92 ms against 1.87).
+    if (reduce_pairs) CURVE_LAUNCH(curve, k_reduce_pairs, nrblocks, REDUCE_BLOCK, 0, st, ra);
+    else CURVE_LAUNCH_PLAIN(curve, k_reduce, nrblocks, REDUCE_BLOCK, 0, st, ra);
     CK_LAUNCH("k_reduce");
     MARK(7);
 
@@ -780,11 +804,11 @@ cudaError_t Plan::run_tail(void *scratch, const u32 *buckets, bool dense, u32 *r
     for (size_t lv = 0; lv + 1 < tree_first.size(); lv++) {
         const u32 cnt = tree_first[lv + 1] - tree_first[lv];
         TreeArgs ta{groups + tree_first[lv], cnt, p.parts, p.parts_s, p.wres};
-        CURVE_LAUNCH(curve, k_reduce_tree, (cnt + TREE_WARPS - 1) / TREE_WARPS, TREE_BLOCK, 0, st, ta);
+        CURVE_LAUNCH(curve, k_reduce_tree, cnt, TREE_BLOCK, 0, st, ta);
         CK_LAUNCH("k_reduce_tree");
     }
     FinalArgs fa2{p.desc, p.wres, M, carry_mode == 0 ? nullptr : p.carry, carry_mode == 2 ? 0 : 1, p.res};
-    CURVE_LAUNCH(curve, k_final, (M + 31) / 32, 32, 0, st, fa2);
+    CURVE_LAUNCH(curve, k_final, M, 32, 0, st, fa2);
     CK_LAUNCH("k_final");
     MARK(8);
     return cudaSuccess;
@@ -1072,12 +1096,12 @@ MsmShape impeller::ctx_shape(const impeller_ctx *ctx, u32 n, u32 c) {
 
 const u32 *impeller::ctx_point_base(const impeller_ctx *ctx) { return ctx->tables ? ctx->tables : ctx->points; }
 
-static Plan *ctx_plan(impeller_ctx *ctx, u32 n, u32 c, bool pairs = true) {
+static Plan *ctx_plan(impeller_ctx *ctx, u32 n, u32 c, bool no_pairs = false) {
     auto key = std::make_pair(n, c);
     auto it = ctx->plans.find(key);
     if (it != ctx->plans.end()) return it->second.get();
     std::unique_ptr<Plan> p(new Plan());
-    if (!Plan::build(*p, ctx->device, {ctx_shape(ctx, n, c)}, pairs)) return nullptr;
+    if (!Plan::build(*p, ctx->device, {ctx_shape(ctx, n, c)}, true, no_pairs)) return nullptr;
     Plan *raw = p.get();
     raw->set_profiling(ctx->profiling);
     ctx->plans[key] = std::move(p);
@@ -1236,7 +1260,7 @@ static cudaError_t ctx_run_locked(impeller_ctx *ctx, const uint32_t *d_scalars, 
         // no room for the affine levels' points: the plan without them
         (void)cudaGetLastError();
         ctx->plans.erase(std::make_pair((u32)n, (u32)c));
-        p = ctx_plan(ctx, (u32)n, c, false);
+        p = ctx_plan(ctx, (u32)n, c, true);
         if (!p) return cudaErrorInvalidValue;
         e = ctx_reserve(ctx, p->scratch_bytes(), stream);
     }
@@ -1368,7 +1392,7 @@ cudaError_t impeller_batch_create(impeller_batch **out, impeller_ctx *ctx, const
     if (e == cudaErrorMemoryAllocation && b->plan.pair_levels) {
         // no room for the affine levels' points: the plan without them
         (void)cudaGetLastError();
-        if (!Plan::build(b->plan, ctx->device, shapes, false)) {
+        if (!Plan::build(b->plan, ctx->device, shapes, true, true)) {
             scratch_release(ctx->device);
             return cudaErrorInvalidValue;
         }

@@ -69,10 +69,13 @@ struct PlanLayout {
 class Plan {
   public:
     // Every MSM reads points[table_base + (w / n_windows) * table_stride + i].
-    // pairs: the plan may add points pairwise in affine form before the
-    // accumulation, where that is faster; it then takes more scratch (the
-    // levels' points).
-    static bool build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool pairs = false);
+    // resident: a plan kept by a context or a batch.  It may add points
+    // pairwise in affine form before the accumulation, where that is faster
+    // (no_pairs: not; the levels' points take scratch), and a single small MSM
+    // takes the one-block sort.  Plans built for a footprint (the server's,
+    // the drop-in call's) keep the layout whose sizes add up over jobs.
+    static bool build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool resident = false,
+                      bool no_pairs = false);
     // Whether a plan of these shapes would sort its entries with the
     // two-level counting sort (fast) rather than the per-entry atomic sort
     // that build() falls back to for very large batches.
@@ -148,6 +151,7 @@ class Plan {
     u32 pair_levels = 0;  // k_affine_pairs levels before the accumulation
     u32 phi_base = 0, phi_points = 0;  // endomorphism images: first virtual index, points (0: none)
     u32 hist_grid_x = 1;
+    bool reduce_pairs = false;  // k_reduce_pairs instead of k_reduce
     // two-level sort (msd) or per-entry atomic bucket sort
     bool msd = false;
     bool small_sort = false;  // k_small_sort instead of either

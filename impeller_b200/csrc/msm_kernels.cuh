@@ -31,6 +31,7 @@
 #include "affine_pairs.cuh"
 #include "bn254.cuh"
 #include "glv.cuh"
+#include "lane_pairs.cuh"
 #include "launch.cuh"
 
 namespace impeller {
@@ -213,7 +214,7 @@ __device__ __forceinline__ u32 block_scan_excl(u32 v, u32 &total, u32 *warp_tot)
 template <class C, bool GLV>
 __global__ void __launch_bounds__(SMALL_SORT_BLOCK)
 k_small_sort(const MsmDesc *__restrict__ descs, const u32 *only_scalars, u32 nb, u32 *__restrict__ offsets,
-             u32 *__restrict__ entries, u32 *__restrict__ long_list) {
+             u32 *__restrict__ entries, u32 *__restrict__ run_counts) {
     grid_wait();
     extern __shared__ u32 cur[];  // nb
     __shared__ u32 warp_tot[32];
@@ -221,7 +222,7 @@ k_small_sort(const MsmDesc *__restrict__ descs, const u32 *only_scalars, u32 nb,
     const u32 *const scalars = only_scalars ? only_scalars : d.scalars;
     const u32 B = 1u << (d.c - 1), t = threadIdx.x;
     for (u32 b = t; b < nb; b += SMALL_SORT_BLOCK) cur[b] = 0;
-    if (t == 0) long_list[0] = 0;
+    if (t < 2) run_counts[t] = 0;
     __syncthreads();
     auto digits = [&](auto &&emit) {
         for (u32 i = t; i < d.n; i += SMALL_SORT_BLOCK) {
@@ -898,12 +899,14 @@ struct FixupArgs {
     const u32 *offsets;
     u32 nb;
     u32 T;               // accumulate threads
-    const u32 *rec_bucket;
-    const u32 *rec_point;
+    u32 *rec_bucket;
+    u32 *rec_point;
     u32 *buckets;
     u32 *long_list;      // [0] = count, then owner thread ids
     u32 long_cap;
     u32 warp_max;        // longest run k_fixup_long gives one warp (0: every run)
+    u32 *wide_count;     // longer ones: their number (zero at launch)
+    u32 *wide_list;      // and owner thread ids (at most T / warp_max)
 };
 
 // Owner of a cut bucket = the slice where the bucket begins (record 2t+1).
@@ -919,6 +922,10 @@ __global__ void k_fixup_short(FixupArgs f) {
     const u32 E = f.offsets[f.nb];
     const u32 L = (E + f.T - 1) / f.T;
     const u32 t1 = (f.offsets[b + 1] - 1) / L;
+    if (f.warp_max && t1 - t + 1 > f.warp_max) {
+        f.wide_list[atomicAdd(f.wide_count, 1u)] = t;
+        return;
+    }
     if (t1 - t > 4) {
         u32 k = atomicAdd(&f.long_list[0], 1u);
         if (k < f.long_cap) f.long_list[1 + k] = t;
@@ -929,66 +936,127 @@ __global__ void k_fixup_short(FixupArgs f) {
     xyzz_store(f.buckets + (size_t)b * C::XW, acc);
 }
 
-// Long runs (a bucket spread over more than 5 slices), in one launch:
-// blocks below wide_blocks take the runs of more than warp_max pieces, one
-// 128-thread block per run (every thread one piece, more only past 128;
-// then a warp sum and a sum of the warps' sums: log2 of the run's length
-// deep); the other blocks' warps take the shorter runs, one warp per run
-// (pieces / 32 additions per lane, then a 5-step warp sum).  Both kinds run
-// at the same time.  wide_blocks == 0 or warp_max == 0: every run by a warp.
-static constexpr u32 WIDE_BLOCK = 128;
+// Long runs (a bucket spread over more than 5 slices; k_fixup_short lists
+// them), in one launch: blocks below wide_blocks take the runs of more than
+// warp_max pieces in parts of
+// WIDE_PART pieces, one 128-thread block per part (up to eight pieces a thread,
+// then a warp sum and a sum of the warps' sums; with parts of 512 or 256 the
+// runs of mid-size MSMs no longer fit one round of blocks); the block that finishes a run's last
+// part adds the parts' sums in the same way.  The other blocks' warps take the
+// shorter runs, one warp per run (16 lane pairs: pieces / 16 additions per
+// pair, then a 4-step sum).  Both kinds run at the same time.
+// warp_max == 0 (and wide_blocks == 0): every run by a warp.
+// Skewed 2^20 points, runs of some 3000 pieces: both fixups 0.28 ms with one
+// block per run, 0.21 ms so.
+static constexpr u32 WIDE_BLOCK = 128, WIDE_PART = 1024;
 template <class C>
 __global__ void k_fixup_long(FixupArgs f, u32 wide_blocks) {
     grid_wait();
     using FQ = typename C::Fq;
-    __shared__ __align__(16) u32 part[WIDE_BLOCK / 32][C::XW];
+    __shared__ __align__(16) u32 part_sum[WIDE_BLOCK / 32][C::XW];
     const u32 lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     const u32 count = min(f.long_list[0], f.long_cap);
     const u32 E = f.offsets[f.nb];
     const u32 L = (E + f.T - 1) / f.T;
-    const u32 wmax = f.warp_max && wide_blocks ? f.warp_max : 0xffffffffu;
     if (blockIdx.x < wide_blocks) {
-        for (u32 w = blockIdx.x; w < count; w += wide_blocks) {  // the same runs for the whole block
-            const u32 t = f.long_list[1 + w];
-            const u32 b = f.rec_bucket[2 * t + 1];
-            const u32 pieces = (f.offsets[b + 1] - 1) / L - t + 1;  // the owner's, then slices t+1 ..
-            if (pieces <= wmax) continue;
-            XyzzT<FQ> acc = xyzz_identity<FQ>();
-            for (u32 k = threadIdx.x; k < pieces; k += WIDE_BLOCK) {
-                const size_t slot = k == 0 ? 2 * (size_t)t + 1 : 2 * (size_t)(t + k);
-                acc = xyzz_add(acc, xyzz_load<FQ>(f.rec_point + slot * C::XW));
+        __shared__ u32 last_part, run_t[WIDE_BLOCK], run_b[WIDE_BLOCK], run_pieces[WIDE_BLOCK];
+        const u32 wide = *f.wide_count;
+        u32 item = 0;  // parts of all runs, in list order; every wide_blocks-th is this block's
+        for (u32 w = 0; w < wide; w++) {
+            if (w % WIDE_BLOCK == 0) {  // the next runs of the list, one per thread
+                __syncthreads();
+                if (w + threadIdx.x < wide) {
+                    const u32 t = f.wide_list[w + threadIdx.x];
+                    const u32 b = f.rec_bucket[2 * t + 1];
+                    run_t[threadIdx.x] = t;
+                    run_b[threadIdx.x] = b;
+                    // the owner's piece, then slices t + 1 ..
+                    run_pieces[threadIdx.x] = (f.offsets[b + 1] - 1) / L - t + 1;
+                }
+                __syncthreads();
             }
-            const u32 nw = min((pieces + 31) / 32, WIDE_BLOCK / 32);  // warps holding pieces
-            if (wid < nw) {
+            const u32 t = run_t[w % WIDE_BLOCK], b = run_b[w % WIDE_BLOCK], pieces = run_pieces[w % WIDE_BLOCK];
+            const u32 parts = (pieces + WIDE_PART - 1) / WIDE_PART;
+            const auto slot = [&](u32 k) { return k == 0 ? 2 * (size_t)t + 1 : 2 * (size_t)(t + k); };
+            for (u32 part = (blockIdx.x + wide_blocks - item % wide_blocks) % wide_blocks; part < parts; part += wide_blocks) {
+                // the sum of `n` points, point k at record slot(k0 + k step)
+                const auto block_sum = [&](u32 k0, u32 step, u32 n) {
+                    XyzzT<FQ> acc = xyzz_identity<FQ>();
+                    for (u32 k = threadIdx.x; k < n; k += WIDE_BLOCK)
+                        acc = xyzz_add(acc, xyzz_load<FQ>(f.rec_point + slot(k0 + k * step) * C::XW));
+                    const u32 nw = min((n + 31) / 32, WIDE_BLOCK / 32);  // warps holding points
+                    if (wid < nw) {
 #pragma unroll 1
-                for (u32 o = 16; o; o >>= 1) acc = xyzz_add(acc, xyzz_shfl_down(acc, o));
-                if (lane == 0) xyzz_store(&part[wid][0], acc);
-            }
-            __syncthreads();
-            if (wid == 0) {
-                XyzzT<FQ> v = lane < nw ? xyzz_load<FQ>(&part[lane][0]) : xyzz_identity<FQ>();
-                u32 P = 1;
-                while (P < nw) P <<= 1;
+                        for (u32 o = 16; o; o >>= 1) acc = xyzz_add(acc, xyzz_shfl_down(acc, o));
+                        if (lane == 0) xyzz_store(&part_sum[wid][0], acc);
+                    }
+                    __syncthreads();
+                    if (wid == 0) {
+                        acc = lane < nw ? xyzz_load<FQ>(&part_sum[lane][0]) : xyzz_identity<FQ>();
+                        u32 P = 1;
+                        while (P < nw) P <<= 1;
 #pragma unroll 1
-                for (u32 o = P >> 1; o; o >>= 1) v = xyzz_add(v, xyzz_shfl_down(v, o));
-                if (lane == 0) xyzz_store(f.buckets + (size_t)b * C::XW, v);
+                        for (u32 o = P >> 1; o; o >>= 1) acc = xyzz_add(acc, xyzz_shfl_down(acc, o));
+                    }
+                    return acc;  // in thread 0
+                };
+                const u32 k0 = part * WIDE_PART;
+                XyzzT<FQ> acc = block_sum(k0, 1, min(WIDE_PART, pieces - k0));
+                if (parts == 1) {
+                    if (threadIdx.x == 0) xyzz_store(f.buckets + (size_t)b * C::XW, acc);
+                    __syncthreads();  // part_sum is reused
+                    continue;
+                }
+                // A part's sum takes the place of its first piece; the block
+                // that finishes the run's last part adds the parts.  They are
+                // counted in the record word of the run's second slice, which
+                // holds b and has no other reader.
+                if (threadIdx.x == 0) {
+                    xyzz_store(f.rec_point + slot(k0) * C::XW, acc);
+                    __threadfence();
+                    last_part = atomicAdd(&f.rec_bucket[2 * (t + 1)], 1u) == b + parts - 1;
+                }
+                __syncthreads();
+                if (last_part) {
+                    __threadfence();
+                    acc = block_sum(0, WIDE_PART, parts);
+                    if (threadIdx.x == 0) xyzz_store(f.buckets + (size_t)b * C::XW, acc);
+                }
+                __syncthreads();  // part_sum and last_part are reused
             }
-            __syncthreads();  // part is reused by the block's next run
+            item += parts;
         }
         return;
     }
     const u32 nwarps = ((gridDim.x - wide_blocks) * blockDim.x) >> 5;
+    const u32 idx = lane >> 1;
+    const bool odd = lane & 1u;
     for (u32 w = ((blockIdx.x - wide_blocks) * blockDim.x + threadIdx.x) >> 5; w < count; w += nwarps) {
         const u32 t = f.long_list[1 + w];
         const u32 b = f.rec_bucket[2 * t + 1];
-        const u32 t1 = (f.offsets[b + 1] - 1) / L;
-        if (t1 - t + 1 > wmax) continue;  // a wide block's
-        XyzzT<FQ> acc = xyzz_identity<FQ>();
-        if (lane == 0) acc = xyzz_load<FQ>(f.rec_point + (size_t)(2 * t + 1) * C::XW);
-        for (u32 s = t + 1 + lane; s <= t1; s += 32)
-            acc = xyzz_add(acc, xyzz_load<FQ>(f.rec_point + (size_t)(2 * s) * C::XW));
+        const u32 pieces = (f.offsets[b + 1] - 1) / L - t + 1;  // the owner's, then slices t + 1 ..
+        // 16 lane pairs: piece k to pair k mod 16, then a sum over the pairs
+        const auto piece = [&](u32 k) {
+            if (k >= pieces) return xyzz_identity<FQ>();
+            const size_t slot = k == 0 ? 2 * (size_t)t + 1 : 2 * (size_t)(t + k);
+            return xyzz_load<FQ>(f.rec_point + slot * C::XW);
+        };
+        XyzzT<FQ> acc = piece(idx);
+        const u32 rounds = (pieces + 15) / 16 - 1;
+        u32 P = 1;
+        while (P < min(pieces, 16u)) P <<= 1;
+        u32 o = P;
 #pragma unroll 1
-        for (u32 o = 16; o; o >>= 1) acc = xyzz_add(acc, xyzz_shfl_down(acc, o));
+        for (u32 k = 1; k <= rounds || o > 1; k++) {
+            XyzzT<FQ> q;
+            if (k <= rounds) {
+                q = piece(16 * k + idx);
+            } else {
+                o >>= 1;
+                q = xyzz_shfl_down(acc, 2 * o);
+            }
+            acc = xyzz_add_pair(acc, q, odd, 0xffffffffu);
+        }
         if (lane == 0) xyzz_store(f.buckets + (size_t)b * C::XW, acc);
     }
 }
@@ -1085,6 +1153,64 @@ __global__ void __launch_bounds__(REDUCE_BLOCK, C::XW == 32 ? REDUCE_BLOCKS_PER_
     Xz v = xyzz_add<FQ, ReduceMul>(sos, ex);
 #pragma unroll 1
     for (u32 o = 16; o; o >>= 1) v = xyzz_add<FQ, ReduceMul>(v, xyzz_shfl_down(v, o));
+    if (lane == 0) {
+        const size_t slot = (size_t)(wd.part_base + blk.y * REDUCE_WARPS + wid) * C::XW;
+        xyzz_store(r.parts_v + slot, v);
+        xyzz_store(r.parts_s + slot, x);
+    }
+}
+
+// The same with two lanes per chunk of buckets, 16 chunks per warp: for plans of
+// up to REDUCE_PAIRS_MAX buckets, whose time is the chain of additions and not
+// their number.  One copy of the addition, in a loop.
+static constexpr u32 REDUCE_PAIRS_MAX = 1u << 17;
+template <class C>
+__global__ void __launch_bounds__(REDUCE_BLOCK) k_reduce_pairs(ReduceArgs r) {
+    grid_wait();
+    using FQ = typename C::Fq;
+    using Xz = XyzzT<FQ>;
+    const uint2 blk = r.blocks[blockIdx.x];
+    const WinDesc wd = r.wins[blk.x];
+    const u32 lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, idx = lane >> 1;
+    const bool odd = lane & 1u;
+    const u32 j = (blk.y * REDUCE_BLOCK + threadIdx.x) >> 1;
+    const u32 lo = j * wd.chunk;  // weights lo + 1 .. lo + chunk
+    const auto bucket = [&](u32 k) {  // of weight lo + k
+        const u32 g = wd.bucket_base + lo + k - 1;
+        if (lo + k > wd.nbuckets || !(r.dense || r.offsets[g + 1] != r.offsets[g])) return xyzz_identity<FQ>();
+        return xyzz_load<FQ>(r.buckets + (size_t)g * C::XW);
+    };
+    // x: running sum from the top, v: sum of the running sums (2 (chunk - 1)
+    // steps); then x: inclusive suffix sums over the warp (4 steps), v: plus
+    // chunk times the exclusive suffix (1), and the sum of v (4)
+    Xz x = bucket(wd.chunk), v = x;
+    const u32 serial = 2 * (wd.chunk - 1);
+#pragma unroll 1
+    for (u32 step = 0; step < serial + 9; step++) {
+        const u32 s = step - serial;
+        Xz p = v, q;
+        u32 o = 0;
+        bool to_x = false;
+        if (step < serial) {
+            to_x = !(step & 1u);
+            if (to_x) p = x;
+            q = to_x ? bucket(wd.chunk - 1 - step / 2) : x;
+        } else if (s < 4) {
+            o = 1u << s;
+            p = x;
+            q = xyzz_shfl_down(x, 2 * o);
+            to_x = true;
+        } else if (s == 4) {
+            q = xyzz_shfl_down(x, 2);
+            if (idx == 15) q = xyzz_identity<FQ>();
+            q = xyzz_dbl_n_pair(q, ilog2(wd.chunk), odd, 0xffffffffu);
+        } else {
+            q = xyzz_shfl_down(v, 2 * (8u >> (s - 5)));
+        }
+        const Xz t = xyzz_add_pair(p, q, odd, 0xffffffffu);
+        if (!to_x) v = t;
+        else if (idx + o < 16) x = t;
+    }
     if (lane == 0) {
         const size_t slot = (size_t)(wd.part_base + blk.y * REDUCE_WARPS + wid) * C::XW;
         xyzz_store(r.parts_v + slot, v);
@@ -1200,8 +1326,7 @@ struct TreeGroup {
     u32 shift;     // log2 K of the input level
 };
 static constexpr u32 TREE_FINAL = 0x80000000u;
-static constexpr u32 TREE_BLOCK = 128;
-static constexpr u32 TREE_WARPS = TREE_BLOCK / 32;
+static constexpr u32 TREE_BLOCK = 64;  // 32 lane pairs
 
 struct TreeArgs {
     const TreeGroup *groups;  // this level's groups
@@ -1211,51 +1336,83 @@ struct TreeArgs {
     u32 *wres;                // window totals
 };
 
+// One block per group, one lane pair per partial (two warps of 16 pairs).  All
+// point additions are one copy of the code in a loop: it stays in the
+// instruction cache, where straight-line copies stream through it.
 template <class C>
-__global__ void __launch_bounds__(TREE_BLOCK, C::XW == 32 ? 2 : 1) k_reduce_tree(TreeArgs a) {
+__global__ void __launch_bounds__(TREE_BLOCK) k_reduce_tree(TreeArgs a) {
     grid_wait();
     using FQ = typename C::Fq;
     using Xz = XyzzT<FQ>;
-    const u32 g = blockIdx.x * TREE_WARPS + (threadIdx.x >> 5);
-    if (g >= a.count) return;  // whole warps leave together
-    const u32 lane = threadIdx.x & 31u;
-    const TreeGroup gr = a.groups[g];
-    Xz A = xyzz_identity<FQ>(), x = xyzz_identity<FQ>();
-    if (lane < gr.in_count) {
-        A = xyzz_load<FQ>(a.parts_v + (size_t)(gr.in_base + lane) * C::XW);
-        x = xyzz_load<FQ>(a.parts_s + (size_t)(gr.in_base + lane) * C::XW);
-    }
-    // Lanes at or above in_count hold the identity; P, the next power of two
-    // at or above in_count, bounds every step below (a window's last group
-    // is often small).
+    __shared__ __align__(16) u32 sm[2][16][C::XW];
+    const u32 lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, i = lane >> 1, idx = wid * 16 + i;
+    const bool odd = lane & 1u;
+    const TreeGroup gr = a.groups[blockIdx.x];
+    const bool two = gr.in_count > 16;  // partials in both warps
+    // Pairs at or above in_count hold the identity; P, the next power of two at
+    // or above in_count (at most 16), bounds the steps inside a warp.
     u32 P = 1;
-    while (P < gr.in_count) P <<= 1;
-    // inclusive suffix sums of S
+    while (P < min(gr.in_count, 16u)) P <<= 1;
+    Xz x = xyzz_identity<FQ>(), v = x;
+    if (idx < gr.in_count) x = xyzz_load<FQ>(a.parts_s + (size_t)(gr.in_base + idx) * C::XW);
 #pragma unroll 1
-    for (u32 o = 1; o < P; o <<= 1) {
-        Xz y = xyzz_shfl_down(x, o);
-        if (lane + o < 32) x = xyzz_add<FQ, TailMul>(x, y);
-    }
-    Xz w = lane ? x : xyzz_identity<FQ>();
-    // The sums of A and of w over the group: the first step folds lanes l
-    // and l + P/2 so that lanes below P/2 carry partial sums of A and lanes
-    // P/2 .. P-1 of w, then each half reduces on its own -- one addition per
-    // step, not two.  Lane 0 ends with the sum of A, lane P/2 with that of w.
-    const u32 half = P >> 1;
-    Xz v = A;
-    if (half) {
-        v = xyzz_add<FQ, TailMul>(lane < half ? A : w, xyzz_shfl_xor(lane < half ? w : A, half));
-#pragma unroll 1
-        for (u32 o = half >> 1; o; o >>= 1) v = xyzz_add<FQ, TailMul>(v, xyzz_shfl_xor(v, o));
-    }
-    if (lane == half && half) v = xyzz_dbl_n<FQ, TailMul>(v, gr.shift);
-    w = half ? xyzz_shfl_down(v, half) : xyzz_identity<FQ>();
-    if (lane == 0) {
-        A = xyzz_add<FQ, TailMul>(v, w);
-        if (gr.out & TREE_FINAL) {
-            xyzz_store(a.wres + (size_t)(gr.out & ~TREE_FINAL) * C::XW, A);
+    for (u32 step = 0; step < 11; step++) {
+        Xz p, q;
+        u32 o = 0;
+        if (step < 4) {  // inclusive suffix sums of S inside the warp
+            o = 1u << step;
+            if (o >= P) continue;
+            p = x;
+            q = xyzz_shfl_down(x, 2 * o);
+        } else if (step == 4) {  // the first warp's suffixes go on over the second's
+            if (!two) continue;
+            if (threadIdx.x == 32) xyzz_store(&sm[0][0][0], x);
+            __syncthreads();
+            p = x;
+            q = xyzz_load<FQ>(&sm[0][0][0]);
+            __syncthreads();
+        } else if (step == 5) {
+            // From here the first warp sums A and the second the weighted S:
+            // they trade the halves of the other's sum that they hold.
+            const Xz A = idx < gr.in_count ? xyzz_load<FQ>(a.parts_v + (size_t)(gr.in_base + idx) * C::XW)
+                                           : xyzz_identity<FQ>();
+            const Xz w = idx ? x : xyzz_identity<FQ>();
+            if (!odd) xyzz_store(&sm[wid][i][0], wid ? A : w);
+            __syncthreads();
+            q = xyzz_load<FQ>(&sm[wid ^ 1u][i][0]);
+            __syncthreads();
+            p = wid ? w : A;
+            v = wid ? q : A;
+            if (!two) continue;  // the second warp has none of its own
+        } else if (step < 10) {  // each warp's sum
+            o = 8u >> (step - 6);
+            if (o >= P) continue;
+            p = v;
+            q = xyzz_shfl_down(v, 2 * o);
+        } else {  // sum of A + K (weighted sum of S)
+            if (wid) {
+                v = xyzz_dbl_n_pair(v, gr.shift, odd, 0xffffffffu);
+                if (lane == 0) xyzz_store(&sm[0][0][0], v);
+            }
+            __syncthreads();
+            if (wid) return;
+            p = v;
+            q = xyzz_load<FQ>(&sm[0][0][0]);
+        }
+        const Xz r = xyzz_add_pair(p, q, odd, 0xffffffffu);
+        if (step < 4) {
+            if (i + o < 16) x = r;
+        } else if (step == 4) {
+            if (!wid) x = r;
         } else {
-            xyzz_store(a.parts_v + (size_t)gr.out * C::XW, A);
+            v = r;
+        }
+    }
+    if (lane == 0) {
+        if (gr.out & TREE_FINAL) {
+            xyzz_store(a.wres + (size_t)(gr.out & ~TREE_FINAL) * C::XW, v);
+        } else {
+            xyzz_store(a.parts_v + (size_t)gr.out * C::XW, v);
             xyzz_store(a.parts_s + (size_t)gr.out * C::XW, x);
         }
     }
@@ -1270,25 +1427,31 @@ struct FinalArgs {
     u32 *results;     // one affine point (C::PW words) per MSM
 };
 
-// One thread per MSM: Horner over its windows, sum_w 2^(c w) T_w with
-// c * (windows - 1) doublings (in Jacobian form between the additions),
-// then the carry and the affine form.
+// One lane pair per MSM (and one MSM per warp): Horner over its windows,
+// sum_w 2^(c w) T_w with c * (windows - 1) doublings (in Jacobian form between
+// the additions), then the carry and the affine form.
 template <class C>
 __global__ void k_final(FinalArgs f) {
     grid_wait();
     using FQ = typename C::Fq;
-    const u32 m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= f.M) return;
+    const u32 m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (m >= f.M || (threadIdx.x & 31u) > 1) return;
+    const bool odd = threadIdx.x & 1u;
+    constexpr u32 mask = 3;
     const MsmDesc d = f.descs[m];
-    XyzzT<FQ> acc = xyzz_identity<FQ>();
-    for (int w = (int)d.n_windows - 1; w >= 0; w--) {
-        acc = xyzz_dbl_n<FQ, FinalMul>(acc, d.c);
-        acc = xyzz_add<FQ, FinalMul>(acc, xyzz_load<FQ>(f.wres + (size_t)(d.win_base + w) * C::XW));
+    XyzzT<FQ> acc = xyzz_load<FQ>(f.wres + (size_t)(d.win_base + d.n_windows - 1) * C::XW);
+    // the windows below the top one, then the carry
+    const int last = f.carry ? -1 : 0;
+#pragma unroll 1
+    for (int w = (int)d.n_windows - 2; w >= last; w--) {
+        if (w >= 0) acc = xyzz_dbl_n_pair(acc, d.c, odd, mask);
+        const u32 *q = w >= 0 ? f.wres + (size_t)(d.win_base + w) * C::XW : f.carry + (size_t)m * C::XW;
+        acc = xyzz_add_pair(acc, xyzz_load<FQ>(q), odd, mask);
     }
-    if (f.carry) acc = xyzz_add<FQ, FinalMul>(acc, xyzz_load<FQ>(f.carry + (size_t)m * C::XW));
     if (f.emit_affine) {
-        affine_store(f.results + (size_t)m * C::PW, xyzz_to_affine_fast<FQ, FinalMul>(acc));
-    } else {
+        const AffineT<FQ> r = xyzz_to_affine_fast<FQ, FinalMul>(acc);
+        if (!odd) affine_store(f.results + (size_t)m * C::PW, r);
+    } else if (!odd) {
         xyzz_store(f.carry + (size_t)m * C::XW, acc);
     }
 }
