@@ -32,4 +32,23 @@ inline cudaError_t launch_next(void (*kern)(P...), dim3 grid, dim3 block, size_t
     return cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
 
+// The same with the blocks in clusters of `cluster`.
+template <class... P, class... A>
+inline cudaError_t launch_cluster(void (*kern)(P...), dim3 grid, dim3 block, unsigned cluster, cudaStream_t st,
+                                  A... args) {
+    cudaLaunchAttribute at[2]{};
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 }  // namespace impeller

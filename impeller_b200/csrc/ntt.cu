@@ -80,13 +80,12 @@ __device__ __forceinline__ Fe<F> smem_load(const uint4 *s, u32 plane, u32 e) {
 
 __device__ __forceinline__ u32 brev(u32 x, u32 bits) { return bits ? __brev(x) >> (32 - bits) : 0; }
 
-// w^e: from the caller's table (twiddle[e] = w^e), or recomputed from three
+// w^e: recomputed from three
 // power tables tab[t][j] = w^(j << 11t) (one or two extra products).
 // Recomputing transforms of more than one tile keep a fourth table, the roots
 // of order 2^11: tab[3][j] = w^(j << (L - 11)), j < 2^10.
-template <class F, bool RECOMP>
+template <class F>
 __device__ __forceinline__ Fe<F> twiddle(const u32 *tw, u32 e) {
-    if (!RECOMP) return fe_load<F>(tw + 8 * (u64)e);
     Fe<F> w = fe_load<F>(tw + 8 * (e & (TAB - 1)));
     if (e >> TAB_LOG) w = fe_mul<F>(w, fe_load<F>(tw + 8 * (TAB + ((e >> TAB_LOG) & (TAB - 1)))));
     if (e >> (2 * TAB_LOG)) w = fe_mul<F>(w, fe_load<F>(tw + 8 * (2 * TAB + (e >> (2 * TAB_LOG)))));
@@ -104,8 +103,6 @@ __device__ __forceinline__ Fe<F> twiddle(const u32 *tw, u32 e) {
 // kernel at 76-80 registers: three 256-thread CTAs per SM (24 warps), 7.6 %
 // faster at 2^24 than holding all four values in registers (114 registers,
 // two CTAs).
-// rev_out (only when the tile is the whole array): write element p to
-// position rev_L(p), canonical.
 //
 // Recomputed twiddles (RECOMP, several passes): the stage twiddles above are
 // all different, so the pass takes the 2^R-point transforms of its digit with
@@ -116,7 +113,7 @@ __device__ __forceinline__ Fe<F> twiddle(const u32 *tw, u32 e) {
 // of a coset shift multiplied in first: 462 -> 338 us.
 template <class F, bool RECOMP>
 __global__ void __launch_bounds__(THREADS, 3)
-k_ntt_pass(View v, const u32 *tw, u32 L, u32 lo, u32 R, u32 logC, int rev_out) {
+k_ntt_pass(View v, const u32 *tw, u32 L, u32 lo, u32 R, u32 logC) {
     impeller::grid_wait();
     extern __shared__ uint4 ntt_smem[];
     const u32 tile_log = R + logC;
@@ -127,10 +124,10 @@ k_ntt_pass(View v, const u32 *tw, u32 L, u32 lo, u32 R, u32 logC, int rev_out) {
     const u64 low0 = (t & ((1ull << nlb_log) - 1)) << logC;
     const u64 hi = t >> nlb_log;
     const u64 gbase = (hi << (lo + R)) | low0;
-    const bool split = RECOMP && L > TILE_LOG;  // digit roots, then one factor per element
+    constexpr bool split = RECOMP;  // digit roots, then one factor per element
     // twiddle of stage s = lo + sl for d mod 2^sl (of the digit) and the low index
     const auto stage_twiddle = [&](u32 sl, u32 dm, u32 low, bool &one) {
-        if (RECOMP && split) {
+        if (split) {
             const u32 ex = dm << (TILE_LOG - 1 - sl);
             one = ex == 0;
             return ex;
@@ -140,8 +137,7 @@ k_ntt_pass(View v, const u32 *tw, u32 L, u32 lo, u32 R, u32 logC, int rev_out) {
         return ex;
     };
     const auto root = [&](u32 ex) {
-        if (RECOMP && split) return fe_load<F>(tw + 8 * (3 * TAB + (u64)ex));
-        return twiddle<F, RECOMP>(tw, ex);
+        return fe_load<F>(tw + 8 * (split ? 3 * TAB + (u64)ex : (u64)ex));
     };
 
     for (u32 e = threadIdx.x; e < tsize; e += blockDim.x) {
@@ -211,19 +207,12 @@ k_ntt_pass(View v, const u32 *tw, u32 L, u32 lo, u32 R, u32 logC, int rev_out) {
         __syncthreads();
     }
 
-    if (rev_out) {
-        for (u32 e = threadIdx.x; e < tsize; e += blockDim.x) {
-            const Fe<F> a = fe_canon<F>(smem_load<F>(ntt_smem, tsize, e));
-            fe_store(at(v, brev(e, L)), a);
-        }
-        return;
-    }
-    if (RECOMP && split && lo) {
+    if (split && lo) {
         for (u32 e = threadIdx.x; e < tsize; e += blockDim.x) {
             const u32 d = e >> logC, c = e & (C - 1);
             const u32 ex = ((u32)(low0 + c) * brev(d, R)) << (L - lo - R);  // below 2^L
             Fe<F> a = smem_load<F>(ntt_smem, tsize, e);
-            if (ex) a = fe_mul<F>(a, twiddle<F, true>(tw, ex));
+            if (ex) a = fe_mul<F>(a, twiddle<F>(tw, ex));
             fe_store(at(v, gbase | ((u64)d << lo) | c), a);
         }
         return;
@@ -233,6 +222,76 @@ k_ntt_pass(View v, const u32 *tw, u32 L, u32 lo, u32 R, u32 logC, int rev_out) {
         uint4 *p = reinterpret_cast<uint4 *>(at(v, gi));
         p[0] = ntt_smem[e];
         p[1] = ntt_smem[tsize + e];
+    }
+}
+
+// Transforms of at most 2^11 elements: the time is a chain of L products, so the
+// 2^(L-8) blocks of a cluster share the work, 256 elements and one butterfly
+// per thread and stage in each (one block does it all up to 2^8).  Block r
+// takes the elements i = r mod 2^q, so that the stages of the index bits from
+// q = L - 8 up stay inside the block; then the blocks trade elements through
+// one another's shared memory, block r takes indices r 2^8 .. and runs the
+// stages of the low q bits, and writes element i to position rev_L(i),
+// canonical.  2^10 elements: 11.2 us, 18.8 with one block of 256 threads.
+constexpr u32 SMALL_LOG = 8;
+template <class F>
+__global__ void __launch_bounds__(1 << (SMALL_LOG - 1)) k_ntt_small(View v, const u32 *tw, u32 L) {
+    impeller::grid_wait();
+    __shared__ uint4 sm[2][2 << SMALL_LOG];
+    constexpr u32 plane = 1u << SMALL_LOG;
+    const u32 m = L < SMALL_LOG ? L : SMALL_LOG, q = L - m, size = 1u << m;
+    const u32 t = threadIdx.x, r = q ? blockIdx.x : 0;
+    for (u32 k = t; k < size; k += blockDim.x) {
+        const uint4 *p = reinterpret_cast<const uint4 *>(at(v, (k << q) | r));
+        sm[0][k] = p[0];
+        sm[0][plane + k] = p[1];
+    }
+    // one stage: bit sl of the index in s; ex(low) is the exponent for the
+    // index bits below it
+    const auto stage = [&](uint4 *s, u32 sl, u32 shift, u32 low_shift, u32 low_or) {
+        __syncthreads();
+        if (t < size / 2) {
+            const u32 low = t & ((1u << sl) - 1), e0 = ((t >> sl) << (sl + 1)) | low, e1 = e0 + (1u << sl);
+            const u32 ex = ((low << low_shift) | low_or) << shift;
+            const Fe<F> w = fe_load<F>(tw + 8 * (u64)ex);
+            const Fe<F> a = smem_load<F>(s, plane, e0), b = smem_load<F>(s, plane, e1);
+            Fe<F> d = fe_sub<F>(a, b);
+            smem_store<F>(s, plane, e0, fe_add<F>(a, b));
+            if (ex) d = fe_mul<F>(d, w);
+            smem_store<F>(s, plane, e1, d);
+        }
+    };
+#pragma unroll 1
+    for (u32 sl = m; sl-- > 0;) stage(sm[0], sl, L - 1 - (sl + q), q, r);
+    uint4 *s = sm[0];
+    if (q) {
+        // index (r << 8) | k lies in block k mod 2^q, at ((r << 8) | k) >> q
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        s = sm[1];
+        const u32 base = (u32)__cvta_generic_to_shared(&sm[0][0]);
+        for (u32 k = t; k < size; k += blockDim.x) {
+            u32 from;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(from) : "r"(base), "r"(k & ((1u << q) - 1)));
+            const u32 slot = ((r << SMALL_LOG) | k) >> q;
+            uint4 x, y;
+            asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w)
+                         : "r"(from + slot * 16));
+            asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(y.x), "=r"(y.y), "=r"(y.z), "=r"(y.w)
+                         : "r"(from + (plane + slot) * 16));
+            s[k] = x;
+            s[plane + k] = y;
+        }
+        // no block may leave while another still reads its memory
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+#pragma unroll 1
+        for (u32 sl = q; sl-- > 0;) stage(s, sl, L - 1 - sl, 0, 0);
+    }
+    __syncthreads();
+    for (u32 k = t; k < size; k += blockDim.x) {
+        const u32 i = (r << SMALL_LOG) | k;
+        fe_store(at(v, brev(i, L)), fe_canon<F>(smem_load<F>(s, plane, k)));
     }
 }
 
@@ -300,7 +359,7 @@ __global__ void k_pow_tables(const u32 *omegas, u32 *tab, u32 n_omegas, u32 coun
 template <class F>
 __global__ void k_powers(const u32 *tab, u32 *out, u64 len, u64 step) {
     for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (u64)gridDim.x * blockDim.x)
-        fe_store(out + 8 * i, fe_canon<F>(twiddle<F, true>(tab, (u32)(i * step))));
+        fe_store(out + 8 * i, fe_canon<F>(twiddle<F>(tab, (u32)(i * step))));
 }
 
 // poly[i] *= powers[((begin + i) mod plen) mod pnum]
@@ -371,43 +430,51 @@ struct PassPlan {
     u32 lo, R, logC;
 };
 
+// Tile of a transform of more than 2^11 elements.  Tiles of 2^10 elements (128
+// threads, six blocks per SM) keep the multipliers busier than tiles of 2^11
+// (three of 256 threads), as more blocks are between their barriers; they are
+// taken where they neither cost a pass nor cut the global runs below 256
+// bytes.  2^24 elements: 3.74 ms with tiles of 2^11, 3.47 with 2^10.
+u32 tile_log(u32 L) {
+    const u32 np = (L - TILE_LOG + MID_MAX - 1) / MID_MAX, np_small = (L - (TILE_LOG - 1) + MID_MAX - 1) / MID_MAX;
+    const u32 digit = (L - (TILE_LOG - 1) + np_small - 1) / np_small;
+    return np_small == np && digit + 3 <= TILE_LOG - 1 ? TILE_LOG - 1 : TILE_LOG;
+}
+
 std::vector<PassPlan> plan_passes(u32 L) {
     std::vector<PassPlan> p;
-    if (L <= TILE_LOG) {
-        p.push_back({0, L, 0});
-        return p;
-    }
-    const u32 M = L - TILE_LOG;
+    if (L <= TILE_LOG) return p;
+    const u32 tile = tile_log(L), M = L - tile;
     const u32 np = (M + MID_MAX - 1) / MID_MAX;
     u32 cursor = L;
     for (u32 k = 0; k < np; k++) {
         const u32 R = M / np + (k < M % np ? 1 : 0);
         cursor -= R;
-        p.push_back({cursor, R, TILE_LOG - R});
+        p.push_back({cursor, R, tile - R});
     }
-    p.push_back({0, TILE_LOG, 0});
+    p.push_back({0, tile, 0});
     return p;
 }
 
 template <class F, bool RECOMP>
 cudaError_t run_ntt(const View &v, const u32 *tw, u32 L, cudaStream_t st) {
     if (L == 0) return cudaSuccess;
+    if (L <= TILE_LOG) {
+        // both kinds of table start with w^e, e < 2^(L-1)
+        const u32 q = L > SMALL_LOG ? L - SMALL_LOG : 0;
+        impeller::launch_cluster(k_ntt_small<F>, 1u << q, 1u << (SMALL_LOG - 1), 1u << q, st, v, tw, L);
+        return launched("k_ntt_small");
+    }
     auto kern = k_ntt_pass<F, RECOMP>;
     NTT_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE * 32));
-    const std::vector<PassPlan> passes = plan_passes(L);
-    const bool single = L <= TILE_LOG;
-    for (const PassPlan &pp : passes) {
-        const u32 tile_log = pp.R + pp.logC;
-        const u64 grid = 1ull << (L - tile_log);
-        impeller::launch_next(kern, (unsigned)grid, THREADS, (size_t)32 << tile_log, st, v, tw, L, pp.lo, pp.R, pp.logC,
-                              single ? 1 : 0);
+    for (const PassPlan &pp : plan_passes(L)) {
+        const u32 tile = pp.R + pp.logC;
+        impeller::launch_next(kern, (unsigned)(1ull << (L - tile)), 1u << (tile - 3), (size_t)32 << tile, st, v, tw, L,
+                              pp.lo, pp.R, pp.logC);
         NTT_CK(launched("k_ntt_pass"));
     }
-    if (!single) {
-        impeller::launch_next(k_ntt_reverse<F>, 1u << (L - 2 * REV_T), 256, 0, st, v, L);
-        NTT_CK(launched("k_ntt_reverse"));
-    }
-    return cudaSuccess;
+    impeller::launch_next(k_ntt_reverse<F>, 1u << (L - 2 * REV_T), 256, 0, st, v, L);
+    return launched("k_ntt_reverse");
 }
 
 // Power tables of w = omegas[0] (omegas[k] = w^(2^k), n_om of them, device),
@@ -605,7 +672,7 @@ cudaError_t impeller_ntt_distribute_powers(int field, PolyPtr poly, const unsign
 
 unsigned int impeller_ntt_launches(unsigned int log_len) {
     if (log_len == 0) return 0;
-    return (unsigned)plan_passes(log_len).size() + (log_len > TILE_LOG ? 1u : 0u);
+    return log_len > TILE_LOG ? (unsigned)plan_passes(log_len).size() + 1u : 1u;
 }
 
 // The reference's five symbols, on its default field (BN254 Fr).
