@@ -430,12 +430,20 @@ struct PassPlan {
     u32 lo, R, logC;
 };
 
-// Tile of a transform of more than 2^11 elements.  Tiles of 2^10 elements (128
-// threads, six blocks per SM) keep the multipliers busier than tiles of 2^11
-// (three of 256 threads), as more blocks are between their barriers; they are
-// taken where they neither cost a pass nor cut the global runs below 256
-// bytes.  2^24 elements: 3.74 ms with tiles of 2^11, 3.47 with 2^10.
+// Tile of a transform of more than 2^11 elements.
+//
+// Up to 2^20 elements two passes of half of the index bits each: the data lie
+// in L2, so that short runs cost little, and small tiles spread a small
+// transform over the SMs (2^12: 36 -> 20 us against a tile of 2^10, 2^16:
+// 51 -> 37, 2^20: 237 -> 219 against 9 and 11 bits).
+//
+// Above, tiles of 2^10 elements (128 threads, six blocks per SM) keep the
+// multipliers busier than tiles of 2^11 (three of 256 threads), as more blocks
+// are between their barriers; they are taken where they neither cost a pass
+// nor cut the global runs below 256 bytes.  2^24 elements: 3.74 ms with tiles
+// of 2^11, 3.47 with 2^10.
 u32 tile_log(u32 L) {
+    if (L <= 2 * (TILE_LOG - 1)) return L <= 16 ? 8 : (L + 1) / 2;
     const u32 np = (L - TILE_LOG + MID_MAX - 1) / MID_MAX, np_small = (L - (TILE_LOG - 1) + MID_MAX - 1) / MID_MAX;
     const u32 digit = (L - (TILE_LOG - 1) + np_small - 1) / np_small;
     return np_small == np && digit + 3 <= TILE_LOG - 1 ? TILE_LOG - 1 : TILE_LOG;
@@ -445,7 +453,7 @@ std::vector<PassPlan> plan_passes(u32 L) {
     std::vector<PassPlan> p;
     if (L <= TILE_LOG) return p;
     const u32 tile = tile_log(L), M = L - tile;
-    const u32 np = (M + MID_MAX - 1) / MID_MAX;
+    const u32 np = L <= 2 * (TILE_LOG - 1) ? 1 : (M + MID_MAX - 1) / MID_MAX;
     u32 cursor = L;
     for (u32 k = 0; k < np; k++) {
         const u32 R = M / np + (k < M % np ? 1 : 0);
@@ -469,7 +477,9 @@ cudaError_t run_ntt(const View &v, const u32 *tw, u32 L, cudaStream_t st) {
     NTT_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE * 32));
     for (const PassPlan &pp : plan_passes(L)) {
         const u32 tile = pp.R + pp.logC;
-        impeller::launch_next(kern, (unsigned)(1ull << (L - tile)), 1u << (tile - 3), (size_t)32 << tile, st, v, tw, L,
+        // up to 2^17 elements a thread takes one quad of elements a round
+        // instead of two: there are SMs to spare
+        impeller::launch_next(kern, (unsigned)(1ull << (L - tile)), 1u << (tile - (L <= 17 ? 2 : 3)), (size_t)32 << tile, st, v, tw, L,
                               pp.lo, pp.R, pp.logC);
         NTT_CK(launched("k_ntt_pass"));
     }
