@@ -290,14 +290,17 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
     // addition, half the additions at once): L leaves each warp a scheduler of
     // its own.
     p.reduce_pairs = nb <= REDUCE_PAIRS_MAX;
-    const u64 target = p.reduce_pairs ? (u64)sms * 64 : (u64)sms * REDUCE_LANES_PER_SM;
+        const u64 target = p.reduce_pairs ? (u64)sms * 64 : (u64)sms * REDUCE_LANES_PER_SM;
     u32 L = 1;
     while (nb / L > target && L < (1u << 30)) L <<= 1;
     std::vector<uint2> rblocks;
     u32 nparts = 0;
     for (u32 wi = 0; wi < wins.size(); wi++) {
         WinDesc &w = wins[wi];
-        w.chunk = std::min(L, w.nbuckets);
+        // (and a full warp for each window: a batch's small windows would
+        // otherwise be one lane's chain of 2L additions; 64 uneven MSMs:
+        // 30.2 -> 28.9 ms)
+        w.chunk = std::min(L, std::max(1u, w.nbuckets / (p.reduce_pairs ? 16 : 32)));
         const u32 nthreads = (w.nbuckets + w.chunk - 1) / w.chunk * (p.reduce_pairs ? 2 : 1);
         const u32 nblocks = (nthreads + REDUCE_BLOCK - 1) / REDUCE_BLOCK;
         w.part_base = nparts;
