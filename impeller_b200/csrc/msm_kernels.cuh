@@ -2,22 +2,26 @@
 //
 // One pass over a batch of M MSMs that share one device-resident point array:
 //
-//   k_histogram   scalar (Montgomery Fr) -> canonical -> signed c-bit digits;
-//                 count entries per bucket                      [HBM-bound]
-//   k_scan_*      exclusive scan of the bucket counts -> bucket offsets
-//   k_scatter     same digits; place (point index, sign) of every nonzero
-//                 digit into its bucket's slice of `entries`     [HBM-bound]
-//   k_accumulate  persistent threads walk equal slices of `entries`, one
+//   sort          scalar (Montgomery Fr) -> canonical -> signed c-bit digits
+//                 (BN254 without window tables: of the scalar's two halves,
+//                 glv.cuh) -> entries (point index, sign) in bucket order:
+//                 k_small_sort for one small MSM, the two-level counting sort
+//                 (k_coarse_*, k_seg_*, k_bin_scan, k_scan_*), or k_histogram
+//                 and k_scatter for very large batches
+//   k_images      abscissae of the points' images under the endomorphism
+//   k_affine_pairs  levels of pairwise affine additions inside the buckets of
+//                 large MSMs (affine_pairs.cuh)                [IMAD-bound]
+//   k_accumulate  persistent threads walk equal slices of what is left, one
 //                 XYZZ += affine (madd-2008-s) per entry; buckets that fit in
 //                 one slice are written directly, buckets cut by a slice
 //                 boundary leave partial sums                  [IMAD-bound]
 //   k_fixup_*     merge the partial sums of cut buckets (short runs per
-//                 thread, long runs -- heavy buckets -- per warp)
-//   k_reduce      per window sum_k k * S_k by chunked running sums whose
-//                 cross-chunk weights come from a suffix scan
-//   k_window_sum  per window (one warp): finish the window total, weight it
-//                 by 2^(c * window)
-//   k_final       per MSM (one warp): sum the windows, affine conversion
+//                 thread, longer ones per warp, heavy buckets per block or
+//                 several)                                    [latency-bound]
+//   k_reduce, k_reduce_pairs  per window sum_k k * S_k by chunked running sums
+//                 whose cross-chunk weights come from a suffix scan
+//   k_reduce_tree finish the window totals, 32 partials to one per level
+//   k_final       per MSM (two lanes): Horner over the windows, affine form
 //
 // Differences from the reference (core/src/msm/src/msm_impl.cuh): the
 // reference sorts 64-bit keys with CUB radix sort (:459-463), protects the
@@ -1073,7 +1077,7 @@ __global__ void k_fixup_long(FixupArgs f, u32 wide_blocks) {
 // shuffle scan) and log2(L) doublings -- no per-lane scalar multiplication.
 // Each warp leaves V_w = sum over its lanes of (sos_j + L * warp-local
 // suffix_{j+1}) and S_w = sum of its chunk sums; the part owed to later warps
-// of the window is 32 L * sum_w w * S_w, added by k_window_sum.
+// of the window is 32 L * sum_w w * S_w, added by k_reduce_tree.
 
 struct ReduceArgs {
     const WinDesc *wins;
@@ -1085,24 +1089,10 @@ struct ReduceArgs {
     u32 dense;            // 1: every bucket holds a point (identity when empty); ignore offsets
 };
 
-// Products of the reduction-tree levels, which run one to a few dozen
-// warps of straight-line point additions: one out-of-line copy (MulCall),
-// 11 % faster than inlined at 2^19 buckets on B200.  k_final's Horner loop
-// repeats one doubling, whose inlined code stays in the instruction cache:
-// inlined there (8 % faster than out-of-line at window 17).  k_reduce runs
-// a few warps per SM: inlined (out-of-line measured 10-19 % slower).
-#ifndef TAIL_MUL_POLICY
-#define TAIL_MUL_POLICY MulCall
-#endif
-#ifndef FINAL_MUL_POLICY
-#define FINAL_MUL_POLICY MulInline
-#endif
-#ifndef REDUCE_MUL_POLICY
-#define REDUCE_MUL_POLICY MulInline
-#endif
-using TailMul = TAIL_MUL_POLICY;
-using FinalMul = FINAL_MUL_POLICY;
-using ReduceMul = REDUCE_MUL_POLICY;
+// k_reduce runs a few warps per SM: products inlined (out-of-line measured
+// 10-19 % slower), as in the one affine conversion of k_final.
+using FinalMul = MulInline;
+using ReduceMul = MulInline;
 
 static constexpr u32 REDUCE_BLOCK = 128;
 // Two 128-thread CTAs per SM (190 registers, no spills): the reduce grid
@@ -1310,8 +1300,8 @@ __global__ void __launch_bounds__(WSUM_BLOCK) k_window_sum(WindowSumArgs a) {
 // ------------------------------------------------------ reduction tree
 //
 // After k_reduce, window total T = sum_g A_g + K * sum_g g * S_g over the
-// window's partials g (A = V, S of the reduce warps, K = 32 L).  One warp per
-// group of 32 consecutive partials g = 32 r + j folds them into one:
+// window's partials g (A = V, S of the reduce warps, K = 32 L; 16 L after
+// k_reduce_pairs).  One block per group of 32 consecutive partials g = 32 r + j folds them into one:
 //   A'_r = sum_j A_{32r+j} + K * sum_j j * S_{32r+j},   S'_r = sum_j S_{32r+j},
 // so that T = sum_r A'_r + 32 K * sum_r r * S'_r: the same form with K' = 32 K.
 // sum_j j * S_j = sum_{i >= 1} x_i for the inclusive suffix sums x of S.  A

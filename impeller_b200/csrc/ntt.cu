@@ -12,13 +12,13 @@
 //     access is a run of C * 32 B) into shared memory, runs the R radix-2
 //     stages there two at a time (a thread takes four elements through two
 //     stages between shared-memory round trips; one Montgomery product per
-//     butterfly), and writes the tile back in place.  Tiles are disjoint, so passes are in place without
-//     a scratch array.  The last pass takes the lowest 11 bits (a contiguous
-//     2048-element block);
+//     butterfly), and writes the tile back in place.  Tiles are disjoint, so
+//     passes are in place without a scratch array.  The last pass takes the
+//     lowest bits (a contiguous block);
 //   - one reordering pass (index bit reversal) with two 16 x 16 tiles per CTA
 //     (the tile of middle bits b and the tile of rev(b) swap), which also
-//     reduces every value to canonical form.  When n <= 2048 the single tile
-//     of the only pass is written out reversed directly.
+//     reduces every value to canonical form;
+//   - up to 2^11 elements one cluster of blocks does everything.
 // Work per element: L/2 Montgomery products and L additions/subtractions, so
 // on B200 the transform is bound by the integer multiply-add rate (like the
 // MSM's accumulation), not by HBM: a pass moves 64 B per element plus twiddle
