@@ -137,21 +137,36 @@ def signed_digit_stats(scalars_canonical: np.ndarray, c: int, shared: bool = Fal
     return nonzero, (len(used) if shared else buckets)
 
 
-# DRAM bytes per k_accumulate launch, measured with ncu (dram__bytes_read.sum
-# + dram__bytes_write.sum) on the same kernel at n = 2^21 with window tables
-# c = 20 (3.607 GB + 0.071 GB) and scaled to n = 2^22 by the number of
-# entries (traffic grows in proportion): used when the run matches.
-NCU_TRAFFIC_2E22_TABLES_C20 = 7.36e9
-
 # One Fq Montgomery product is 8 rows x (8 products a_j*b_i, 1 for the
 # reduction factor, 8 products m*N_j) = 136 32x32->64-bit partial products; a
 # Montgomery square takes 36 + 8 + 64 = 108 (symmetric cross products).  A
 # mixed XYZZ + affine addition (madd-2008-s) is 8 products and 2 squares:
-# 1304 partial products.
+# 1304 partial products.  An affine addition of the pairwise levels is 5
+# products and 1 square (its share of the inversion counted as products: one
+# going forward, two going backward): 788.  BLS12-381's products are 300
+# partial products each, squares too.
 PRODUCTS_PER_MUL = 136
 PRODUCTS_PER_SQR = 108
-MULS_PER_MADD = 10
 PRODUCTS_PER_MADD = 8 * PRODUCTS_PER_MUL + 2 * PRODUCTS_PER_SQR
+PRODUCTS_PER_PAIR = 5 * PRODUCTS_PER_MUL + PRODUCTS_PER_SQR
+PRODUCTS_PER_MUL_BLS = 300
+
+
+def accumulate_work(entries: float, nonempty: float, buckets: int, sms: int, bls: bool = False) -> dict:
+    """The accumulate phase's additions and partial products on uniform
+    scalars.  Pairwise affine levels run while the buckets hold 8 points and
+    more on average and a level has enough slots (the engine's rule); after k
+    of them a bucket of m points holds ceil(m / 2^k), m / 2^k + (1 - 2^-k) / 2
+    on average, and mixed additions fold these."""
+    k, slots_min = 0, sms * (10240 if bls else 20480)
+    while k < 6 and entries >= 8 * buckets << k and (int(entries) + (2 * (1 << k) - 1) * buckets) >> (k + 1) >= slots_min:
+        k += 1
+    left = entries / (1 << k) + nonempty * (1 - 0.5 ** k) / 2
+    pairs, madds = entries - left, left - nonempty
+    per_pair, per_madd = ((6 * PRODUCTS_PER_MUL_BLS, 10 * PRODUCTS_PER_MUL_BLS) if bls
+                          else (PRODUCTS_PER_PAIR, PRODUCTS_PER_MADD))
+    return {"levels": k, "pair_additions": pairs, "madds": madds, "products_per_pair": per_pair,
+            "products_per_madd": per_madd, "products": pairs * per_pair + madds * per_madd}
 
 
 # ------------------------------------------------------------- reference
@@ -424,19 +439,21 @@ def main():
         canon = [M.to_host(M.gen_scalars_device(n, seed=0, stream_id=1 + v, mont=False, device=dev)).reshape(n, 8)
                  for v in range(V)]
         stats = [signed_digit_stats(cv, c, shared=bool(c_tab)) for cv in canon]
-        madds = statistics.mean(nz - nb for nz, nb in stats)
         entries = statistics.mean(nz for nz, _ in stats)
+        nbk = (1 << (c - 1)) * (1 if c_tab else math.ceil(254 / c))
+        sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        work = accumulate_work(entries, statistics.mean(nb for _, nb in stats), nbk, sms)
+        additions = work["pair_additions"] + work["madds"]
         peak = ctypes.c_double()
         L.check(lib.impeller_imad_peak(dev, ctypes.byref(peak)))
         acc_ms = phase_ms["accumulate"]
-        achieved = madds * PRODUCTS_PER_MADD / (acc_ms * 1e-3) / 1e9
+        achieved = work["products"] / (acc_ms * 1e-3) / 1e9
         hbm_peak = None
         try:
             hbm_peak = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))["hbm_gbs"]
         except Exception:
             hbm_peak = 6650.0
         sort_ms = phase_ms["histogram"] + phase_ms["scan"] + phase_ms["scatter"]
-        nbk = (1 << (c - 1)) * (1 if c_tab else math.ceil(254 / c))
         sort_bytes = 2 * 32 * n + 4 * entries + 3 * 4 * nbk
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -450,13 +467,11 @@ def main():
                        "l2": "inputs > L2: 256 MiB points + 4 rotating 128 MiB scalar vectors"},
             "gpu_launches": args.steps * ctx.launches(n, c),
             "phase_ms": {k: round(v, 4) for k, v in phase_ms.items()},
-            "roofline": {"bound": "imad", "kernel": "k_accumulate", "achieved": achieved, "peak": peak.value,
+            "roofline": {"bound": "imad", "kernel": "k_affine_pairs + k_accumulate" if work["levels"] else "k_accumulate",
+                         "achieved": achieved, "peak": peak.value,
                          "unit": "G 32x32->64 products/s", "frac": achieved / peak.value,
-                         "traffic": NCU_TRAFFIC_2E22_TABLES_C20 if (args.log2n == 22 and c_tab == 20 and c == 20)
-                         else None,
-                         "algorithmic_bytes": madds * (64 + 4),
-                         "per_launch": {"madds": madds, "products_per_madd": PRODUCTS_PER_MADD,
-                                        "madds_per_s": madds / (acc_ms * 1e-3), "ms": acc_ms},
+                         "algorithmic_bytes": additions * (64 + 4),
+                         "per_launch": {**work, "additions_per_s": additions / (acc_ms * 1e-3), "ms": acc_ms},
                          "peak_source": "impeller_imad_peak: independent Fq Montgomery products (4 chains/thread, 136 partial products each), measured live"},
             "clocks": clocks,
         }
@@ -636,14 +651,16 @@ def bls12381_leg(M, dev, n, args, imad_peak: float) -> dict:
     phase_ms = {lib.impeller_phase_name(i).decode(): phases[i] / nr for i in range(8)}
     ctx.close()
     # accumulate-phase roofline: 12-limb Montgomery products (12 rows of
-    # 12 + 1 + 12 partial products = 300) x 10 per mixed addition
+    # 12 + 1 + 12 partial products = 300), 10 per mixed and 6 per pairwise addition
     W = math.ceil(255 / c) + (1 if c in (3, 5, 15, 17) else 0)
     stats = [signed_digit_stats(M.to_host(M.gen_scalars_device(n, seed=0, stream_id=1 + v, mont=False, device=dev,
                                                                 curve=C)).reshape(n, 8), c, shared=bool(c_tab),
                                 windows=W) for v in range(4)]
-    madds = statistics.mean(nz - nb for nz, nb in stats)
+    work = accumulate_work(statistics.mean(nz for nz, _ in stats), statistics.mean(nb for _, nb in stats),
+                           (1 << (c - 1)) * (1 if c_tab else W),
+                           torch.cuda.get_device_properties(dev).multi_processor_count, bls=True)
     acc_ms = phase_ms["accumulate"]
-    achieved = madds * MULS_PER_MADD * 300 / (acc_ms * 1e-3) / 1e9
+    achieved = work["products"] / (acc_ms * 1e-3) / 1e9
     bls_peak = ctypes.c_double()
     L.check(lib.impeller_imad_peak_curve(dev, C, ctypes.byref(bls_peak)))
     # drop-in ABI, host buffers
@@ -668,10 +685,11 @@ def bls12381_leg(M, dev, n, args, imad_peak: float) -> dict:
     return {"workload": f"single BLS12-381 G1 MSM, n=2^{int(math.log2(n))}, window c={c}",
             "window_tables": bool(c_tab), "value": n / (ms * 1e-3), "unit": UNIT, "ms_per_step": ms,
             "phase_ms": {k: round(v, 4) for k, v in phase_ms.items()},
-            "roofline": {"bound": "imad", "kernel": "k_accumulate<Bls12381>", "achieved": achieved,
+            "roofline": {"bound": "imad", "achieved": achieved,
+                         "kernel": ("k_affine_pairs + " if work["levels"] else "") + "k_accumulate<Bls12381>",
                          "peak": bls_peak.value, "unit": "G 32x32->64 products/s",
                          "frac": achieved / bls_peak.value,
-                         "per_launch": {"madds": madds, "products_per_madd": MULS_PER_MADD * 300, "ms": acc_ms},
+                         "per_launch": {**work, "ms": acc_ms},
                          "peak_8limb": imad_peak,
                          "peak_source": "impeller_imad_peak_curve: independent 12-limb BLS12-381 Fq products "
                                         "(4 chains/thread, 300 partial products each), measured live"},
