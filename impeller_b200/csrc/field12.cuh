@@ -50,14 +50,6 @@ __device__ __forceinline__ void add12(u32 (&r)[12], const u32 *a, const u32 *b) 
           "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]), "r"(b[8]), "r"(b[9]), "r"(b[10]), "r"(b[11]));
 }
 
-// r = a + (mask & b) (12 words).
-__device__ __forceinline__ void add12_masked(u32 (&r)[12], const u32 *a, const u32 *b, u32 mask) {
-    u32 t[12];
-#pragma unroll
-    for (int i = 0; i < 12; i++) t[i] = b[i] & mask;
-    add12(r, a, t);
-}
-
 // Rows of the two-accumulator Montgomery product (see bn254.cuh), 12 limbs.
 __device__ __forceinline__ void bn_row_first12(u32 (&x)[12], u32 (&y)[12], const u32 (&a)[12], u32 w) {
     asm(
