@@ -45,7 +45,7 @@ u32 digit_windows(u32 c, u32 curve) {
     return curve == CURVE_BLS12381 ? Bls12381::windows(c) : Bn254::windows(c);
 }
 
-// Launch `kern` instantiated for the plan's curve.
+// Launch `kern`, which starts with grid_wait, instantiated for the plan's curve.
 #define CURVE_LAUNCH(curve_id, kern, grid, block, smem, st, ...)                      \
     do {                                                                               \
         if ((curve_id) == CURVE_BLS12381)                                              \
@@ -54,7 +54,8 @@ u32 digit_windows(u32 c, u32 curve) {
             launch_next(kern<Bn254>, (grid), (block), (smem), (st), __VA_ARGS__);               \
     } while (0)
 
-// The same after the previous kernel has drained.
+// The same after the previous kernel has drained, for kernels without grid_wait
+// too: their callers' streams (the table builds') also carry other threads' MSMs.
 #define CURVE_LAUNCH_PLAIN(curve_id, kern, grid, block, smem, st, ...)                 \
     do {                                                                               \
         if ((curve_id) == CURVE_BLS12381)                                              \
@@ -890,7 +891,7 @@ u32 *Plan::results_ptr(void *scratch) const {
 }
 
 cudaError_t combine_xyzz(const u32 *d_xyzz, u32 k, u32 *d_out, cudaStream_t stream, u32 curve) {
-    CURVE_LAUNCH(curve, k_combine, 1, 32, 0, stream, d_xyzz, k, d_out);
+    CURVE_LAUNCH_PLAIN(curve, k_combine, 1, 32, 0, stream, d_xyzz, k, d_out);
     CK_LAUNCH("k_combine");
     return cudaSuccess;
 }
@@ -952,7 +953,7 @@ __global__ void __launch_bounds__(128) k_precompute(u32 *points, u64 n, u32 shif
 
 cudaError_t precompute_tables(u32 *d_points, u64 n, u32 shift, u32 n_tables, cudaStream_t stream, u32 curve) {
     if (n == 0 || n_tables <= 1) return cudaSuccess;
-    CURVE_LAUNCH(curve, k_precompute, (u32)((n + 127) / 128), 128, 0, stream, d_points, n, shift, n_tables);
+    CURVE_LAUNCH_PLAIN(curve, k_precompute, (u32)((n + 127) / 128), 128, 0, stream, d_points, n, shift, n_tables);
     CK_LAUNCH("k_precompute");
     return cudaSuccess;
 }
