@@ -466,8 +466,7 @@ __host__ __device__ __forceinline__ u32 pair_levels(u64 entries, u64 nb, u64 slo
 // by those they do have (skewed scalars have many zero digits).  out: the
 // bucket starts after the last level; state: the number of levels, then the
 // levels' tile counters.
-__global__ void k_pair_plan(const u32 *__restrict__ offsets, u32 nb, u32 slots_min, u32 most, u32 *__restrict__ out,
-                            u32 *__restrict__ state) {
+__global__ void k_pair_plan(const u32 *offsets, u32 nb, u32 slots_min, u32 most, u32 *out, u32 *state) {
     grid_wait();
     const u32 used = pair_levels(offsets[nb], nb, slots_min, most);
     if (blockIdx.x == 0 && threadIdx.x <= PAIR_MAX_LEVELS) state[threadIdx.x] = threadIdx.x ? 0 : used;

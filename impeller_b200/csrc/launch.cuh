@@ -4,8 +4,14 @@
 // next kernel is only set up once the previous one has drained.  launch_next
 // lets it be set up beside the previous kernel (programmatic stream
 // serialization); grid_wait, the first thing such a kernel does, waits until
-// the previous kernel has completed and its writes are visible, so that the
-// order of all memory accesses is as before.
+// the previous kernel has completed and its writes are visible.  That orders
+// ordinary accesses as a plain launch does.  It does not order loads through
+// the read-only path (__ldg, or const __restrict__ parameters): the compiler
+// may take those ahead of the wait, and the hardware wants their data unwritten
+// from the kernel's start, which now lies before the previous kernel's end.  So
+// such a kernel reads with plain loads whatever a kernel of the chain writes;
+// only inputs that none of them writes (descriptors, the point array) may be
+// const __restrict__.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(SORT_BLOCK, 2) k_coarse_scatter(SortArgs a) {
         for (u32 w0 = 0; w0 < d.n_logical; w0 += KB) {
             u32 key[KB];
 #pragma unroll
-            for (u32 j = 0; j < KB; j++) key[j] = w0 + j < d.n_logical ? __ldg(kw + (size_t)(w0 + j) * tile_n) : NONE;
+            for (u32 j = 0; j < KB; j++) key[j] = w0 + j < d.n_logical ? kw[(size_t)(w0 + j) * tile_n] : NONE;
 #pragma unroll
             for (u32 j = 0; j < KB; j++) {
                 if (key[j] != NONE) {
@@ -535,13 +535,13 @@ __global__ void __launch_bounds__(FINE_BLOCK) k_seg_hist(SortArgs a) {
     const u32 nv = (v1 - v0) >> 3, bd = blockDim.x;
     u32 k = threadIdx.x;
     for (; k + 3 * bd < nv; k += 4 * bd) {
-        const uint4 q0 = __ldg(v + k), q1 = __ldg(v + k + bd), q2 = __ldg(v + k + 2 * bd), q3 = __ldg(v + k + 3 * bd);
+        const uint4 q0 = v[k], q1 = v[k + bd], q2 = v[k + 2 * bd], q3 = v[k + 3 * bd];
         hist8(hist, q0);
         hist8(hist, q1);
         hist8(hist, q2);
         hist8(hist, q3);
     }
-    for (; k < nv; k += bd) hist8(hist, __ldg(v + k));
+    for (; k < nv; k += bd) hist8(hist, v[k]);
     __syncthreads();
     for (u32 f = threadIdx.x; f < FINE; f += blockDim.x) a.seghist[(size_t)blockIdx.x * FINE + f] = hist[f];
 }
@@ -617,12 +617,12 @@ __global__ void __launch_bounds__(FINE_BLOCK) k_seg_scatter(SortArgs a) {
     const u32 nv = (v1 - v0) >> 2, bd = blockDim.x;
     u32 k = threadIdx.x;
     for (; k + bd < nv; k += 2 * bd) {
-        const uint2 f0 = __ldg(vf + k), f1 = __ldg(vf + k + bd);
-        const uint4 e0 = __ldg(ve + k), e1 = __ldg(ve + k + bd);
+        const uint2 f0 = vf[k], f1 = vf[k + bd];
+        const uint4 e0 = ve[k], e1 = ve[k + bd];
         place4(lcur, stage_e, stage_f, f0, e0);
         place4(lcur, stage_e, stage_f, f1, e1);
     }
-    for (; k < nv; k += bd) place4(lcur, stage_e, stage_f, __ldg(vf + k), __ldg(ve + k));
+    for (; k < nv; k += bd) place4(lcur, stage_e, stage_f, vf[k], ve[k]);
     __syncthreads();
     for (u32 s = threadIdx.x; s < total; s += blockDim.x) a.entries[delta[stage_f[s]] + s] = stage_e[s];
 }
@@ -657,7 +657,7 @@ __device__ __forceinline__ u32 block_exclusive_scan(u32 v, u32 &total) {
 }
 
 // counts must be padded to a multiple of SCAN_TILE with zeros.
-__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_reduce(const u32 *__restrict__ counts, u32 *__restrict__ tile_sums) {
+__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_reduce(const u32 *counts, u32 *tile_sums) {
     grid_wait();
     const uint4 *p = reinterpret_cast<const uint4 *>(counts + (size_t)blockIdx.x * SCAN_TILE) + threadIdx.x * 4;
     u32 s = 0;
@@ -673,7 +673,7 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_reduce(const u32 *__restric
 
 // Single block: exclusive scan of the tile sums in place; tile_sums[ntiles]
 // receives the grand total.
-__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_tiles(u32 *__restrict__ tile_sums, u32 ntiles) {
+__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_tiles(u32 *tile_sums, u32 ntiles) {
     grid_wait();
     u32 carry = 0;
     for (u32 base = 0; base < ntiles; base += SCAN_BLOCK) {
@@ -687,9 +687,8 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_tiles(u32 *__restrict__ til
     if (threadIdx.x == 0) tile_sums[ntiles] = carry;
 }
 
-__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_down(const u32 *__restrict__ counts, const u32 *__restrict__ tile_sums,
-                                                   u32 *__restrict__ offsets, u32 *__restrict__ cursor, u32 nb,
-                                                   u32 ntiles) {
+__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_down(const u32 *counts, const u32 *tile_sums, u32 *offsets, u32 *cursor,
+                                                          u32 nb, u32 ntiles) {
     grid_wait();
     const size_t base = (size_t)blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_PER_THREAD;
     const uint4 *p = reinterpret_cast<const uint4 *>(counts + base);
@@ -744,7 +743,7 @@ __device__ __forceinline__ AffineT<typename C::Fq> load_entry_point(const u32 *_
 
 template <class C>
 __device__ __forceinline__ AffineT<typename C::Fq> load_entry_point(const u32 *__restrict__ points, u32 e,
-                                                                    const u32 *__restrict__ phi, u32 phi_base) {
+                                                                    const u32 *phi, u32 phi_base) {
     const u32 *px, *py;
     entry_coordinates<C, true>(points, e, phi, phi_base, px, py);
     AffineT<typename C::Fq> q;

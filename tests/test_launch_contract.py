@@ -62,3 +62,22 @@ def test_kernels_and_launches_are_found():
 def test_chained_kernels_wait_for_their_predecessor_first(name):
     body = KERNELS[name][1].strip()
     assert re.match(r"(?:impeller::)?grid_wait\(\);", body), f"{name} does not start with grid_wait()"
+
+
+# inputs that no kernel of a chain writes
+READ_ONLY = {"descs", "points"}
+
+
+@pytest.mark.parametrize("name", chained())
+def test_chained_kernels_read_with_plain_loads(name):
+    params, body = KERNELS[name]
+    assert "__ldg" not in body and "ld.global.nc" not in body
+    restrict = set(re.findall(r"const\s+\w+\s*\*\s*__restrict__\s*(\w+)", params))
+    assert restrict <= READ_ONLY, f"{name}: {sorted(restrict - READ_ONLY)}"
+
+
+@pytest.mark.parametrize("name", ["msm_kernels.cuh", "affine_pairs.cuh", "lane_pairs.cuh", "bn254.cuh", "ntt.cu"])
+def test_helpers_of_chained_kernels_read_with_plain_loads(name):
+    text = source(name)
+    assert "__ldg" not in text
+    assert set(re.findall(r"const\s+\w+\s*\*\s*__restrict__\s*(\w+)", text)) <= READ_ONLY
