@@ -145,7 +145,7 @@ constexpr u32 PART_STAGES = 2;
 // window has its own bucket set), so a split scalar takes the nearest width
 // that suits its halves.
 std::vector<MsmShape> group_shapes(const Config &cfg, u32 M, u32 n, u32 part_len) {
-    if (cfg.glv) return std::vector<MsmShape>(M, MsmShape{n, split_window(cfg.c), 0, 0, 0, cfg.curve, part_len});
+    if (cfg.glv) return std::vector<MsmShape>(M, MsmShape{n, split_window(cfg.c), 0, 0, 0, cfg.curve, true});
     std::vector<MsmShape> s(M, MsmShape{n, cfg.c, cfg.n_windows, part_len, 0, cfg.curve});
     return s;
 }

@@ -145,13 +145,34 @@ static size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Digits per scalar and bucket sets of a shape.
 static void shape_windows(const MsmShape &s, u32 &digits, u32 &sets) {
-    if (s.phi_base) {
+    if (s.split) {
         sets = glv::windows(s.c);
         digits = 2 * sets;
     } else {
         digits = digit_windows(s.c, s.curve);
         sets = (s.n_windows == 0 || s.n_windows > digits) ? digits : s.n_windows;
     }
+}
+
+// Where the images' virtual indices start: past every point that an MSM reads,
+// its window tables included.  points: images that the split MSMs need.
+static u64 images_base(const std::vector<MsmShape> &shapes, u32 &points) {
+    u64 base = 0;
+    points = 0;
+    for (const MsmShape &s : shapes) {
+        u32 W, nw;
+        shape_windows(s, W, nw);
+        if (s.split) points = std::max(points, s.n);
+        const u64 tables = s.split || !nw ? 1 : (W + nw - 1) / nw;
+        base = std::max(base, (u64)s.table_base + (tables - 1) * s.table_stride + s.n);
+    }
+    return base;
+}
+
+bool Plan::images_fit(const std::vector<MsmShape> &shapes) {
+    u32 points;
+    const u64 base = images_base(shapes, points);
+    return base + points < (1ull << 31);
 }
 
 // The sort-path rule of Plan::build, from the shapes alone.  Each MSM's
@@ -219,33 +240,30 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
     std::vector<WinDesc> wins;
     u64 nb = 0, entries = 0;
     u32 nmax = 0;
-    p.phi_base = p.phi_points = 0;
-    for (u32 m = 0; m < p.M; m++) {
-        const MsmShape &s = shapes[m];
+    for (const MsmShape &s : shapes)
         if (s.c < 3 || s.c > 31) {
             set_error("window size must be in [3, 31]");
             return false;
         }
+    const u64 images = images_base(shapes, p.phi_points);
+    if (images + p.phi_points >= (1ull << 31)) {
+        set_error("point index space (tables x length) exceeds 2^31");
+        return false;
+    }
+    p.phi_base = (u32)images;
+    for (u32 m = 0; m < p.M; m++) {
+        const MsmShape &s = shapes[m];
         u32 W, nw;
         shape_windows(s, W, nw);
         const u32 n_tables = (W + nw - 1) / nw;
-        const u32 stride = s.phi_base ? s.phi_base : s.table_stride;
+        const u32 stride = s.split ? p.phi_base : s.table_stride;
         const u64 B = 1ull << (s.c - 1);
-        const u64 vmax = (u64)s.table_base + (u64)(n_tables - 1) * stride + s.n;
-        if (s.phi_base && (p.curve != CURVE_BN254 || s.table_base || (p.phi_base && p.phi_base != s.phi_base))) {
-            set_error("endomorphism images need BN254, table 0 and one base index");
+        if (s.split && (p.curve != CURVE_BN254 || s.table_base)) {
+            set_error("split scalars need BN254 and table 0");
             return false;
-        }
-        if (s.phi_base) {
-            p.phi_base = s.phi_base;
-            p.phi_points = std::max(p.phi_points, s.n);
         }
         if (n_tables > 1 && stride < s.n) {
             set_error("table stride smaller than the MSM size");
-            return false;
-        }
-        if (vmax >= (1ull << 31)) {
-            set_error("point index space (tables x length) exceeds 2^31");
             return false;
         }
         nb = align_up(nb, FINE);  // every coarse bin of the sort belongs to one MSM
@@ -256,7 +274,7 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
         d.n_logical = W;
         d.n_windows = nw;
         d.table_stride = stride;
-        d.glv = s.phi_base ? 1u : 0u;
+        d.glv = s.split ? 1u : 0u;
         d.bucket_base = (u32)nb;
         d.win_base = (u32)wins.size();
         d.table_base = s.table_base;
@@ -1094,7 +1112,7 @@ MsmShape impeller::ctx_shape(const impeller_ctx *ctx, u32 n, u32 c) {
     MsmShape s{n, c, 0, 0, 0, ctx->curve};
     const u64 have = ctx->tables ? ctx->tables_points : ctx->len;
     if (ctx->curve == CURVE_BN254 && have + n < (1ull << 31) && 2ull * glv::windows(c) * n < 0xffffffffull)
-        s.phi_base = (u32)have;
+        s.split = true;
     return s;
 }
 

@@ -35,10 +35,8 @@ struct MsmShape {
     u32 table_stride;  // points per window table (used when n_windows < digit windows)
     u32 table_base;    // point index of this MSM's table 0
     u32 curve;         // CURVE_BN254 or CURVE_BLS12381
-    // BN254, plain windows: nonzero splits the scalars by the endomorphism
-    // (glv.cuh); the images of the points take the virtual indices from here
-    // on (at least the point array's length; the same for every MSM of a plan).
-    u32 phi_base = 0;
+    // BN254, plain windows: the scalars are split by the endomorphism (glv.cuh).
+    bool split = false;
 };
 
 // Signed-digit windows of width c for the curve's scalars: the fewest that
@@ -80,6 +78,9 @@ class Plan {
     // two-level counting sort (fast) rather than the per-entry atomic sort
     // that build() falls back to for very large batches.
     static bool two_level_sort(const std::vector<MsmShape> &shapes);
+    // Whether the points and the images of a plan of these shapes together stay
+    // within 31-bit indices (build() refuses it otherwise).
+    static bool images_fit(const std::vector<MsmShape> &shapes);
     ~Plan();
 
     // Enqueue one run.  scalars[m] are device pointers.  carry_mode:
@@ -149,7 +150,9 @@ class Plan {
     u32 accum_blocks = 0, accum_block = 256;
     u32 nparts = 0, long_cap = 0;
     u32 pair_levels = 0;  // k_affine_pairs levels before the accumulation
-    u32 phi_base = 0, phi_points = 0;  // endomorphism images: first virtual index, points (0: none)
+    // Endomorphism images (phi_points of them, 0: none) take virtual indices
+    // from phi_base on, past every point that an MSM of the plan reads.
+    u32 phi_base = 0, phi_points = 0;
     u32 hist_grid_x = 1;
     bool reduce_pairs = false;  // k_reduce_pairs instead of k_reduce
     // two-level sort (msd) or per-entry atomic bucket sort

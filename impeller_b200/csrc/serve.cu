@@ -190,9 +190,10 @@ void dispatcher(impeller_server *s) {
                 Job &j = s->jobs[s->pending.front()];
                 if (s->used + bytes + j.bytes > s->budget) break;
                 // keep the batch on the two-level sort: a batch past its
-                // limits sorts entry by entry, slower than its jobs alone
+                // limits sorts entry by entry, slower than its jobs alone;
+                // and within the index range that its jobs have alone
                 shapes.push_back(j.shape);
-                if (!js.empty() && !Plan::two_level_sort(shapes)) {
+                if (!js.empty() && !(Plan::two_level_sort(shapes) && Plan::images_fit(shapes))) {
                     shapes.pop_back();
                     break;
                 }

@@ -147,3 +147,24 @@ def test_server_setup_failure_releases_and_recovers(M, srs, step, what):
     srv.close()
     ctx.close()
 
+
+
+def test_jobs_around_added_window_tables(M, srs):
+    # plain jobs wait while tables are added, jobs on the tables and plain ones
+    # follow: batches may mix all three kinds
+    ctx = M.MsmContext(srs)
+    sizes = [20000, 3000, 1 << 15, 700, 9000, 1 << 15, 150, 25000]
+    scal = [O.gen_scalars(n, seed=41, stream=i) for i, n in enumerate(sizes)]
+    srv = M.MsmServer(ctx, max_batch=8, max_inflight=1)
+    ids = [(i, srv.submit(scal[i])) for _ in range(6) for i in range(len(sizes))]
+    for c in sorted({M.table_window(n) for n in sizes} - {0}):
+        ctx.precompute(c)
+        ids += [(i, srv.submit(scal[i])) for _ in range(3) for i in range(len(sizes))]
+    res = [(i, srv.wait(j)[0]) for i, j in ids]
+    st = srv.stats()
+    srv.close()
+    want = [O.msm(srs[:n], s) for n, s in zip(sizes, scal)]
+    for i, got in res:
+        assert (got == want[i]).all(), sizes[i]
+    assert st["failed"] == 0
+    ctx.close()

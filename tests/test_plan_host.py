@@ -1,0 +1,88 @@
+"""Plans of MSMs, built on the CPU: a small C++ program links the library, lays
+plans out as its callers do, and the sizes and index ranges are checked.  No
+GPU is needed (the layout assumes 148 SMs where there is no device).
+"""
+import os
+import shutil
+import subprocess
+import tempfile
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+PKG = os.path.join(HERE, "..", "impeller_b200")
+CUDA = os.path.dirname(os.path.dirname(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"))
+
+SOURCE = r"""
+#include <cstdio>
+#include <cstring>
+#include "engine.h"
+using namespace impeller;
+
+// A context of len points as impeller_ctx_create makes it, without a device.
+struct Context {
+    impeller_ctx ctx;
+    explicit Context(u64 len, u32 curve = CURVE_BN254) {
+        ctx.len = len;
+        ctx.curve = curve;
+    }
+    // what impeller_ctx_precompute changes
+    void add_tables(u32 c) {
+        const u64 have = ctx.tables ? ctx.tables_points : ctx.len;
+        ctx.tables = reinterpret_cast<u32 *>(16);
+        ctx.tables_points = have + (u64)digit_windows(c, ctx.curve) * ctx.len;
+        ctx.sets.emplace_back(c, (u32)have);
+    }
+};
+
+static int mixed_batch() {
+    // a plain job, then tables, then a job on the tables and a plain one: what
+    // a server holds when tables are added between its jobs' submissions
+    Context k(5000);
+    const MsmShape before = ctx_shape(&k.ctx, 3000, 13);
+    k.add_tables(16);
+    const MsmShape table = ctx_shape(&k.ctx, 5000, 16), after = ctx_shape(&k.ctx, 2000, 13);
+    Plan p, q, r;
+    const bool one = Plan::build(p, 0, {before, table}), two = Plan::build(q, 0, {before, after});
+    const bool all = Plan::build(r, 0, {after, table, before});
+    const u64 past_table = table.table_base + (u64)(digit_windows(16) - 1) * table.table_stride + table.n;
+    std::printf("built %d %d %d\n", one, two, all);
+    std::printf("images_past_points %d %d %d\n", p.phi_base >= past_table, q.phi_base >= 3000, r.phi_base >= past_table);
+    std::printf("images %u %u %u\n", p.phi_points, q.phi_points, r.phi_points);
+    return 0;
+}
+
+int main(int argc, char **argv) {
+    if (argc > 1 && !std::strcmp(argv[1], "mixed_batch")) return mixed_batch();
+    return 2;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def plans():
+    from impeller_b200 import build
+    gxx = shutil.which("g++")
+    if gxx is None or not os.path.isdir(os.path.join(CUDA, "include")):
+        pytest.skip("g++ or the CUDA headers are not available")
+    build.build()
+    d = tempfile.mkdtemp(prefix="plans_")
+    src, exe = os.path.join(d, "plans.cpp"), os.path.join(d, "plans")
+    with open(src, "w") as f:
+        f.write(SOURCE)
+    subprocess.run([gxx, "-O1", "-std=c++17", "-I", os.path.join(PKG, "csrc"), "-I", os.path.join(CUDA, "include"), src,
+                    "-o", exe, build.LIB, "-Wl,-rpath," + os.path.abspath(PKG), "-lpthread"], check=True)
+
+    def run(what):
+        r = subprocess.run([exe, what], capture_output=True, text=True, timeout=600, check=True)
+        return dict(line.split(" ", 1) for line in r.stdout.splitlines())
+    return run
+
+
+def test_images_lie_past_every_point_of_a_batch(plans):
+    """Virtual indices of endomorphism images must not meet real ones, whatever
+    the context held when a job's shape was made, and no such mix is refused."""
+    r = plans("mixed_batch")
+    assert r["built"] == "1 1 1"
+    assert r["images_past_points"] == "1 1 1"
+    assert r["images"] == "3000 3000 3000"
