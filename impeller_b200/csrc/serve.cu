@@ -131,8 +131,13 @@ cudaError_t launch_batch(impeller_server *s, Batch &b, std::vector<Job *> &js, u
         off += js[m]->n * 8;
     }
     u32 *d_res = reinterpret_cast<u32 *>(base + o_res);
-    if ((e = b.plan->enqueue(base + o_plan, ctx_point_base(s->ctx), sc.data(), d_res, 0, b.stream)) != cudaSuccess)
-        return e;
+    {
+        // a table build in another thread frees the previous tables, after
+        // waiting for what has been launched on them
+        std::lock_guard<std::mutex> g(s->ctx->mu);
+        e = b.plan->enqueue(base + o_plan, ctx_point_base(s->ctx), sc.data(), d_res, 0, b.stream);
+    }
+    if (e != cudaSuccess) return e;
     if ((e = cudaMemcpyAsync(b.h_results, d_res, (size_t)M * RB, cudaMemcpyDeviceToHost, b.stream)) != cudaSuccess)
         return e;
     if ((e = cudaEventRecord(b.ev, b.stream)) != cudaSuccess) return e;
@@ -375,8 +380,11 @@ cudaError_t impeller_server_submit(impeller_server *s, const uint32_t *h_scalars
     Job j;
     j.h_scalars = h_scalars;
     j.n = n;
-    j.c = ctx_window(s->ctx, n);
-    j.shape = ctx_shape(s->ctx, (u32)n, j.c);
+    {
+        std::lock_guard<std::mutex> g(s->ctx->mu);  // the table sets may be growing
+        j.c = ctx_window(s->ctx, n);
+        j.shape = ctx_shape(s->ctx, (u32)n, j.c);
+    }
     Plan p;
     if (!Plan::build(p, s->ctx->device, {j.shape})) return cudaErrorInvalidValue;
     j.bytes = up256(n * 32) + 256 + p.scratch_bytes();
