@@ -1,5 +1,6 @@
 // MSM engine: plan layout, launch sequence, resident-SRS contexts, batches.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -124,6 +125,12 @@ void scratch_release(int device) {
         cudaMemPoolTrimTo(p.pool, 0);
     }
 }
+
+// Test hook: the next of these steps fails (0: none).
+enum : u32 { STEP_SCRATCH = 1, STEP_UPLOAD = 2 };
+static std::atomic<u32> g_fail_step{0};
+
+static bool fail_injected(u32 step) { return g_fail_step.compare_exchange_strong(step, 0u); }
 
 cudaError_t scratch_alloc(void **out, size_t bytes, int device, cudaStream_t st) {
     cudaMemPool_t pool;
@@ -880,12 +887,19 @@ cudaError_t Plan::run_one(void *scratch, const u32 *points, const u32 *scalars, 
         CK(cudaStreamIsCapturing(st, &cap));
         // memory allocated in a capture would belong to its graph
         if (cap != cudaStreamCaptureStatusNone) return enqueue(scratch, points, &scalars, results, 0, st);
-        cudaError_t e = scratch_alloc(&image, tables.size(), device, st);
+        void *d = nullptr;
+        cudaError_t e = scratch_alloc(&d, tables.size(), device, st);
+        if (e == cudaSuccess) {
+            e = fail_injected(STEP_UPLOAD)
+                    ? cudaErrorMemoryAllocation
+                    : cudaMemcpyAsync(d, tables.data(), tables.size(), cudaMemcpyHostToDevice, st);
+            if (e != cudaSuccess) cudaFreeAsync(d, st);
+        }
         if (e != cudaSuccess) {
-            image = nullptr;
+            set_error(std::string("upload of a plan's tables: ") + cudaGetErrorString(e));
             return e;
         }
-        CK(cudaMemcpyAsync(image, tables.data(), tables.size(), cudaMemcpyHostToDevice, st));
+        image = d;
     }
     cudaError_t e = run_front(scratch, points, st, false, image, nullptr, nullptr, scalars);
     if (e != cudaSuccess) return e;
@@ -1207,6 +1221,15 @@ cudaError_t impeller_ctx_create_curve(impeller_ctx **out, int device, const uint
     return cudaSuccess;
 }
 
+cudaError_t impeller_fail_scratch_step(uint32_t step) {
+    if (step > 2) {
+        set_error("impeller_fail_scratch_step: steps are 1 and 2 (0 clears)");
+        return cudaErrorInvalidValue;
+    }
+    g_fail_step.store(step);
+    return cudaSuccess;
+}
+
 cudaError_t impeller_ctx_destroy(impeller_ctx *ctx) {
     if (!ctx) return cudaSuccess;
     cudaSetDevice(ctx->device);
@@ -1289,8 +1312,11 @@ static cudaError_t ctx_run_locked(impeller_ctx *ctx, const uint32_t *d_scalars, 
     if (e != cudaSuccess) return e;
     CK(cudaStreamWaitEvent(stream, ctx->done, 0));
     e = p->run_one(ctx->scratch, ctx_point_base(ctx), d_scalars, d_result, stream);
+    // also after an error: what did get enqueued uses the scratch and the
+    // plan's tables, which the next run may read on another stream
+    const cudaError_t rec = cudaEventRecord(ctx->done, stream);
     if (e != cudaSuccess) return e;
-    CK(cudaEventRecord(ctx->done, stream));
+    CK(rec);
     return cudaSuccess;
 }
 

@@ -110,6 +110,10 @@ cudaError_t impeller_ctx_create(impeller_ctx **out, int device, const uint32_t *
 cudaError_t impeller_ctx_create_curve(impeller_ctx **out, int device, const uint32_t *points, uint64_t len,
                                       int points_on_device, unsigned int curve);
 cudaError_t impeller_ctx_destroy(impeller_ctx *ctx);
+/* Test hook: the next time a context does step `step` (1 its scratch
+ * allocation, 2 the upload of a plan's tables; 0 clears) the step fails with
+ * cudaErrorMemoryAllocation before it runs. */
+cudaError_t impeller_fail_scratch_step(uint32_t step);
 /* Device pointer of the resident points (len x 16 uint32; len x 24 on
  * BLS12-381). */
 const uint32_t *impeller_ctx_points(const impeller_ctx *ctx);
