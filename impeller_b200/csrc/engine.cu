@@ -138,10 +138,13 @@ cudaError_t scratch_alloc(void **out, size_t bytes, int device, cudaStream_t st)
         std::lock_guard<std::mutex> g(g_pool_mu);
         pool = g_pools[device].pool;
     }
+    if (fail_injected(STEP_SCRATCH)) return cudaErrorMemoryAllocation;
     cudaError_t e = cudaMallocFromPoolAsync(out, bytes, pool, st);
     if (e == cudaErrorMemoryAllocation) {
-        // freed pieces may be in the way of a larger one
+        // freed pieces may be in the way of a larger one, until their frees
+        // have run and the pool has given them back
         (void)cudaGetLastError();
+        if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
         cudaMemPoolTrimTo(pool, 0);
         e = cudaMallocFromPoolAsync(out, bytes, pool, st);
     }
@@ -1113,6 +1116,7 @@ static cudaError_t ctx_reserve(impeller_ctx *ctx, size_t bytes, cudaStream_t st)
     if (ctx->scratch) CK(cudaFreeAsync(ctx->scratch, st));
     ctx->scratch = nullptr;
     ctx->scratch_bytes = 0;
+    ctx->resizes++;
     CK(scratch_alloc(&ctx->scratch, bytes, ctx->device, st));
     ctx->scratch_bytes = bytes;
     return cudaSuccess;
@@ -1135,6 +1139,12 @@ const u32 *impeller::ctx_point_base(const impeller_ctx *ctx) { return ctx->table
 static Plan *ctx_plan(impeller_ctx *ctx, u32 n, u32 c, bool no_pairs = false) {
     auto key = std::make_pair(n, c);
     auto it = ctx->plans.find(key);
+    // A plan that took the place of one there was no room for holds until the
+    // scratch is resized again (which waited for its last run).
+    if (it != ctx->plans.end() && it->second->reduced_at && it->second->reduced_at != ctx->resizes) {
+        ctx->plans.erase(it);
+        it = ctx->plans.end();
+    }
     if (it != ctx->plans.end()) return it->second.get();
     std::unique_ptr<Plan> p(new Plan());
     if (!Plan::build(*p, ctx->device, {ctx_shape(ctx, n, c)}, true, no_pairs)) return nullptr;
@@ -1300,14 +1310,17 @@ static cudaError_t ctx_run_locked(impeller_ctx *ctx, const uint32_t *d_scalars, 
     CK(cudaSetDevice(ctx->device));
     Plan *p = ctx_plan(ctx, (u32)n, c);
     if (!p) return cudaErrorInvalidValue;
+    const size_t had = ctx->scratch_bytes;
     cudaError_t e = ctx_reserve(ctx, p->scratch_bytes(), stream);
     if (e == cudaErrorMemoryAllocation && p->pair_levels) {
-        // no room for the affine levels' points: the plan without them
+        // no room for the affine levels' points: the plan without them, in no
+        // less scratch than there was, so that other sizes find theirs
         (void)cudaGetLastError();
         ctx->plans.erase(std::make_pair((u32)n, (u32)c));
         p = ctx_plan(ctx, (u32)n, c, true);
         if (!p) return cudaErrorInvalidValue;
-        e = ctx_reserve(ctx, p->scratch_bytes(), stream);
+        e = ctx_reserve(ctx, std::max(had, p->scratch_bytes()), stream);
+        p->reduced_at = ctx->resizes;
     }
     if (e != cudaSuccess) return e;
     CK(cudaStreamWaitEvent(stream, ctx->done, 0));
@@ -1448,6 +1461,7 @@ cudaError_t impeller_batch_create(impeller_batch **out, impeller_ctx *ctx, const
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // any stream may run the batch
     if (e != cudaSuccess) {
+        if (b->scratch) cudaFreeAsync(b->scratch, nullptr);
         scratch_release(ctx->device);
         set_error(std::string("impeller_batch_create: scratch: ") + cudaGetErrorString(e));
         return e;
@@ -1459,7 +1473,7 @@ cudaError_t impeller_batch_create(impeller_batch **out, impeller_ctx *ctx, const
 
 cudaError_t impeller_batch_destroy(impeller_batch *b) {
     if (!b) return cudaSuccess;
-    cudaSetDevice(b->ctx->device);
+    cudaSetDevice(b->device);
     cudaDeviceSynchronize();
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->g) cudaGraphDestroy(b->g);

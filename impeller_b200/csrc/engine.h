@@ -150,6 +150,7 @@ class Plan {
     u32 accum_blocks = 0, accum_block = 256;
     u32 nparts = 0, long_cap = 0;
     u32 pair_levels = 0;  // k_affine_pairs levels before the accumulation
+    u64 reduced_at = 0;   // impeller_ctx::resizes when there was no room for the plan it stands for (0: none)
     // Endomorphism images (phi_points of them, 0: none) take virtual indices
     // from phi_base on, past every point that an MSM of the plan reads.
     u32 phi_base = 0, phi_points = 0;
@@ -222,6 +223,7 @@ struct impeller_ctx {
     std::mutex mu;
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
+    impeller::u64 resizes = 0;  // of the scratch
     impeller::u32 *d_scalars = nullptr;  // staging for impeller_msm_host
     impeller::u64 d_scalars_cap = 0;
     impeller::u32 *d_result = nullptr;

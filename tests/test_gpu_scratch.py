@@ -37,3 +37,48 @@ def test_run_after_a_failed_upload_of_the_tables(M):
     got = M.to_host(ctx.msm_device(d_sc))
     ctx.close()
     assert np.array_equal(got, O.msm(pts, sc))
+
+
+# 2^18 + 5 points at 64 digits lay out two levels of pairwise additions
+N, C = (1 << 18) + 5, 4
+
+
+@pytest.fixture(scope="module")
+def leveled():
+    pts, sc = O.gen_points(N, seed=22), O.gen_scalars(N, seed=22, stream=1)
+    small = O.gen_scalars(900, seed=22, stream=2)
+    return pts, sc, O.msm(pts, sc), small, O.msm(pts[:900], small)
+
+
+def test_plan_without_levels_takes_over_until_the_scratch_grows(M, leveled):
+    pts, sc, want, small, want_small = leveled
+    d_sc, d_small, ctx = M.to_device(sc), M.to_device(small), M.MsmContext(pts)
+    full = ctx.launches(N, C)
+    assert np.array_equal(M.to_host(ctx.msm_device(d_small, c=8)), want_small)  # some scratch is there
+    fail_next(M, SCRATCH)
+    assert np.array_equal(M.to_host(ctx.msm_device(d_sc, c=C)), want)
+    reduced = ctx.launches(N, C)
+    assert reduced < full
+    # other sizes leave it in place, and it them
+    assert np.array_equal(M.to_host(ctx.msm_device(d_small, c=8)), want_small)
+    assert ctx.launches(N, C) == reduced
+    # a plan that needs more scratch: room again, and the levels are back
+    assert np.array_equal(M.to_host(ctx.msm_device(d_sc, c=3)), want)
+    assert ctx.launches(N, C) == full
+    assert np.array_equal(M.to_host(ctx.msm_device(d_sc, c=C)), want)
+    ctx.close()
+
+
+def test_batch_without_room_for_levels(M, leveled):
+    pts, sc, want, small, want_small = leveled
+    ctx = M.MsmContext(pts)
+    full = ctx.batch([N, 900], windows=[C, 8])
+    fail_next(M, SCRATCH)
+    b = ctx.batch([N, 900], windows=[C, 8])
+    assert b.launches() < full.launches()
+    for batch in (b, full):
+        got = M.to_host(batch.run([M.to_device(sc), M.to_device(small)]))
+        assert np.array_equal(got[0], want) and np.array_equal(got[1], want_small)
+        batch.close()
+    ctx.close()
+
