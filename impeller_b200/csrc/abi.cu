@@ -528,10 +528,10 @@ cudaError_t impeller_msm_cfg_curve(unsigned int curve, unsigned int window_size,
         return cudaErrorInvalidValue;
     }
     if (curve == CURVE_BN254 && cfg.n_tables == 1) {
-        // the halves' digits and the images' indices have to fit 32 bits
+        // (the images take as many indices as the points)
         const u64 per_card = (len + num_cards - 1) / num_cards, part = (per_card + parts - 1) / parts;
-        cfg.glv = 2 * part < (1ull << 31) &&
-                  2ull * ((128 + split_window(cfg.c) - 1) / split_window(cfg.c)) * batch_per_run * part < 0xffffffffull;
+        cfg.glv = 2 * part < (1ull << 31) && split_fits(part, cfg.c, batch_per_run) &&
+                  split_fits(part, split_window(cfg.c), batch_per_run);
     }
     std::vector<CardLayout> layouts(num_cards);
     for (u32 i = 0; i < num_cards; i++) {

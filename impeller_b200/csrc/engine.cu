@@ -1078,6 +1078,15 @@ u32 split_window(u32 c) {
     return best;
 }
 
+// Splitting takes up to a tenth more digits (the halves' windows round up
+// twice) and half the buckets.  It is left out where it would change which
+// sizes are accepted: the digits have to fit 32 bits, and so do the buckets of
+// whole scalars.
+bool split_fits(u64 n, u32 c, u64 msms) {
+    return c >= 3 && c <= 31 && 2 * glv::windows(c) * n * msms < 0xffffffffull &&
+           ((u64)digit_windows(c) << (c - 1)) * msms < (1ull << 31);
+}
+
 // Window of the resident tables the table recommends for MSMs of n points
 // (0: plain windows are faster at that size).
 u32 table_window(u64 n) {
@@ -1100,13 +1109,20 @@ u32 impeller::ctx_set_base(const impeller_ctx *ctx, u32 c) {
     return NONE;
 }
 
+// Whether the context splits the scalars of an MSM over n of its points with
+// plain windows of width c.
+static bool ctx_splits(const impeller_ctx *ctx, u64 n, u32 c) {
+    const u64 have = ctx->tables ? ctx->tables_points : ctx->len;
+    return ctx->curve == CURVE_BN254 && have + n < (1ull << 31) && split_fits(n, c, 1);
+}
+
 // With resident tables the context uses them for the sizes whose best
 // (measured) tables window is one of the sets it holds; other sizes run plain.
-u32 impeller::ctx_window(const impeller_ctx *ctx, u64 n) {
+u32 impeller::ctx_window(const impeller_ctx *ctx, u64 n, bool whole) {
     const u32 ct = table_window(n);
     if (ct && ctx_set_base(ctx, ct) != NONE) return ct;
-    const u32 c = default_window(n);
-    return ctx->curve == CURVE_BN254 ? split_window(c) : curve_window(c, ctx->curve);
+    const u32 c = curve_window(default_window(n), ctx->curve), cs = split_window(c);
+    return !whole && ctx_splits(ctx, n, cs) ? cs : c;
 }
 
 static cudaError_t ctx_reserve(impeller_ctx *ctx, size_t bytes, cudaStream_t st) {
@@ -1124,19 +1140,19 @@ static cudaError_t ctx_reserve(impeller_ctx *ctx, size_t bytes, cudaStream_t st)
 
 // Shape of an MSM of n points with window c on this context: with a resident
 // table set for c every digit window shares one bucket set.
-MsmShape impeller::ctx_shape(const impeller_ctx *ctx, u32 n, u32 c) {
+MsmShape impeller::ctx_shape(const impeller_ctx *ctx, u32 n, u32 c, bool whole) {
     const u32 base = ctx_set_base(ctx, c);
     if (base != NONE) return MsmShape{n, c, 1, (u32)ctx->len, base, ctx->curve};
-    MsmShape s{n, c, 0, 0, 0, ctx->curve};
-    const u64 have = ctx->tables ? ctx->tables_points : ctx->len;
-    if (ctx->curve == CURVE_BN254 && have + n < (1ull << 31) && 2ull * glv::windows(c) * n < 0xffffffffull)
-        s.split = true;
-    return s;
+    return MsmShape{n, c, 0, 0, 0, ctx->curve, !whole && ctx_splits(ctx, n, c)};
 }
 
 const u32 *impeller::ctx_point_base(const impeller_ctx *ctx) { return ctx->tables ? ctx->tables : ctx->points; }
 
-static Plan *ctx_plan(impeller_ctx *ctx, u32 n, u32 c, bool no_pairs = false) {
+// What a plan may leave out where there is no room for it.
+enum PlanKind { PLAN_FULL, PLAN_NO_LEVELS, PLAN_WHOLE_SCALARS };
+
+// whole_c: window of the plan that does not split the scalars
+static Plan *ctx_plan(impeller_ctx *ctx, u32 n, u32 c, PlanKind kind = PLAN_FULL, u32 whole_c = 0) {
     auto key = std::make_pair(n, c);
     auto it = ctx->plans.find(key);
     // A plan that took the place of one there was no room for holds until the
@@ -1147,7 +1163,9 @@ static Plan *ctx_plan(impeller_ctx *ctx, u32 n, u32 c, bool no_pairs = false) {
     }
     if (it != ctx->plans.end()) return it->second.get();
     std::unique_ptr<Plan> p(new Plan());
-    if (!Plan::build(*p, ctx->device, {ctx_shape(ctx, n, c)}, true, no_pairs)) return nullptr;
+    const bool whole = kind == PLAN_WHOLE_SCALARS;
+    if (!Plan::build(*p, ctx->device, {ctx_shape(ctx, n, whole ? whole_c : c, whole)}, true, kind != PLAN_FULL))
+        return nullptr;
     Plan *raw = p.get();
     raw->set_profiling(ctx->profiling);
     ctx->plans[key] = std::move(p);
@@ -1306,18 +1324,21 @@ static cudaError_t ctx_run_locked(impeller_ctx *ctx, const uint32_t *d_scalars, 
         return cudaErrorInvalidValue;
     }
     if (n == 0) return cudaMemsetAsync(d_result, 0, (size_t)point_words(ctx->curve) * 4, stream);
+    const u32 whole_c = c ? c : ctx_window(ctx, n, true);
     if (c == 0) c = ctx_window(ctx, n);
     CK(cudaSetDevice(ctx->device));
     Plan *p = ctx_plan(ctx, (u32)n, c);
     if (!p) return cudaErrorInvalidValue;
     const size_t had = ctx->scratch_bytes;
     cudaError_t e = ctx_reserve(ctx, p->scratch_bytes(), stream);
-    if (e == cudaErrorMemoryAllocation && p->pair_levels) {
-        // no room for the affine levels' points: the plan without them, in no
-        // less scratch than there was, so that other sizes find theirs
+    while (e == cudaErrorMemoryAllocation && (p->pair_levels || p->phi_points)) {
+        // no room for the affine levels' points, then none for the images: the
+        // plan without them, in no less scratch than there was, so that other
+        // sizes find theirs
+        const PlanKind kind = p->pair_levels ? PLAN_NO_LEVELS : PLAN_WHOLE_SCALARS;
         (void)cudaGetLastError();
         ctx->plans.erase(std::make_pair((u32)n, (u32)c));
-        p = ctx_plan(ctx, (u32)n, c, true);
+        p = ctx_plan(ctx, (u32)n, c, kind, whole_c);
         if (!p) return cudaErrorInvalidValue;
         e = ctx_reserve(ctx, std::max(had, p->scratch_bytes()), stream);
         p->reduced_at = ctx->resizes;
@@ -1433,27 +1454,33 @@ cudaError_t impeller_batch_create(impeller_batch **out, impeller_ctx *ctx, const
         set_error("impeller_batch_create: bad argument");
         return cudaErrorInvalidValue;
     }
-    std::vector<MsmShape> shapes;
-    for (u32 i = 0; i < count; i++) {
+    for (u32 i = 0; i < count; i++)
         if (sizes[i] > ctx->len || sizes[i] == 0) {
             set_error("impeller_batch_create: size 0 or larger than the resident point array");
             return cudaErrorInvalidValue;
         }
-        u32 c = windows && windows[i] ? windows[i] : ctx_window(ctx, sizes[i]);
-        shapes.push_back(ctx_shape(ctx, (u32)sizes[i], c));
-    }
     std::unique_ptr<impeller_batch> b(new impeller_batch());
     b->ctx = ctx;
     b->device = ctx->device;
-    if (!Plan::build(b->plan, ctx->device, shapes, true)) return cudaErrorInvalidValue;
+    const auto build = [&](PlanKind kind) {
+        const bool whole = kind == PLAN_WHOLE_SCALARS;
+        std::vector<MsmShape> shapes;
+        for (u32 i = 0; i < count; i++) {
+            const u32 c = windows && windows[i] ? windows[i] : ctx_window(ctx, sizes[i], whole);
+            shapes.push_back(ctx_shape(ctx, (u32)sizes[i], c, whole));
+        }
+        return Plan::build(b->plan, ctx->device, shapes, true, kind != PLAN_FULL);
+    };
+    // (the halves' digits of many MSMs may pass 32 bits where those of whole scalars do not)
+    if (!build(PLAN_FULL) && !build(PLAN_WHOLE_SCALARS)) return cudaErrorInvalidValue;
     CK(cudaSetDevice(ctx->device));
     CK(scratch_hold(ctx->device));
     b->held = true;
     cudaError_t e = scratch_alloc(&b->scratch, b->plan.scratch_bytes(), ctx->device, nullptr);
-    if (e == cudaErrorMemoryAllocation && b->plan.pair_levels) {
-        // no room for the affine levels' points: the plan without them
+    while (e == cudaErrorMemoryAllocation && (b->plan.pair_levels || b->plan.phi_points)) {
+        // no room for the affine levels' points, then none for the images
         (void)cudaGetLastError();
-        if (!Plan::build(b->plan, ctx->device, shapes, true, true)) {
+        if (!build(b->plan.pair_levels ? PLAN_NO_LEVELS : PLAN_WHOLE_SCALARS)) {
             scratch_release(ctx->device);
             return cudaErrorInvalidValue;
         }

@@ -47,6 +47,7 @@ u32 digit_windows(u32 c, u32 curve = CURVE_BN254);
 u32 default_window(u64 n);  // autotune table (or the cost model)
 u32 table_window(u64 n);    // tables window the autotune table recommends (0: none)
 u32 split_window(u32 c);    // c moved off widths whose top digit of a split BN254 scalar is short
+bool split_fits(u64 n, u32 c, u64 msms);  // whether msms BN254 MSMs of n points may split their scalars
 u32 curve_window(u32 c, u32 curve);  // c moved off windows that need an extra digit window on the curve
 
 // Device property cache.
@@ -241,7 +242,8 @@ struct impeller_ctx {
 
 namespace impeller {
 u32 ctx_set_base(const impeller_ctx *ctx, u32 c);            // NONE if no set for c
-u32 ctx_window(const impeller_ctx *ctx, u64 n);              // window an MSM of n points uses
-MsmShape ctx_shape(const impeller_ctx *ctx, u32 n, u32 c);   // plan shape on this context
+// window an MSM of n points uses (whole: without splitting its scalars)
+u32 ctx_window(const impeller_ctx *ctx, u64 n, bool whole = false);
+MsmShape ctx_shape(const impeller_ctx *ctx, u32 n, u32 c, bool whole = false);  // plan shape on this context
 const u32 *ctx_point_base(const impeller_ctx *ctx);          // points (and table sets) base
 }  // namespace impeller

@@ -380,14 +380,18 @@ cudaError_t impeller_server_submit(impeller_server *s, const uint32_t *h_scalars
     Job j;
     j.h_scalars = h_scalars;
     j.n = n;
-    {
-        std::lock_guard<std::mutex> g(s->ctx->mu);  // the table sets may be growing
-        j.c = ctx_window(s->ctx, n);
-        j.shape = ctx_shape(s->ctx, (u32)n, j.c);
+    // whole scalars where the split ones' images do not fit the budget
+    for (const bool whole : {false, true}) {
+        {
+            std::lock_guard<std::mutex> g(s->ctx->mu);  // the table sets may be growing
+            j.c = ctx_window(s->ctx, n, whole);
+            j.shape = ctx_shape(s->ctx, (u32)n, j.c, whole);
+        }
+        Plan p;
+        if (!Plan::build(p, s->ctx->device, {j.shape})) return cudaErrorInvalidValue;
+        j.bytes = up256(n * 32) + 256 + p.scratch_bytes();
+        if (j.bytes <= s->budget || !j.shape.split) break;
     }
-    Plan p;
-    if (!Plan::build(p, s->ctx->device, {j.shape})) return cudaErrorInvalidValue;
-    j.bytes = up256(n * 32) + 256 + p.scratch_bytes();
     std::lock_guard<std::mutex> g(s->mu);
     if (j.bytes > s->budget) {
         s->rejected++;

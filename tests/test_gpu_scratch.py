@@ -75,10 +75,30 @@ def test_batch_without_room_for_levels(M, leveled):
     full = ctx.batch([N, 900], windows=[C, 8])
     fail_next(M, SCRATCH)
     b = ctx.batch([N, 900], windows=[C, 8])
-    assert b.launches() < full.launches()
+    assert b.launches < full.launches
     for batch in (b, full):
         got = M.to_host(batch.run([M.to_device(sc), M.to_device(small)]))
         assert np.array_equal(got[0], want) and np.array_equal(got[1], want_small)
         batch.close()
     ctx.close()
 
+
+
+def test_whole_scalars_where_the_images_find_no_room(M):
+    n = 5000
+    pts, sc = O.gen_points(n, seed=23), O.gen_scalars(n, seed=23, stream=1)
+    want = O.msm(pts, sc)
+    ctx = M.MsmContext(pts)
+    full, d_sc = ctx.launches(n, 13), M.to_device(sc)
+    fail_next(M, SCRATCH)
+    for c in (13, 0):
+        assert np.array_equal(M.to_host(ctx.msm_device(d_sc, c=c)), want)
+    assert ctx.launches(n, 13) == full - 1  # no kernel for the images
+    fail_next(M, SCRATCH)
+    b = ctx.batch([n, 777, 1])
+    for _ in range(2):
+        got = M.to_host(b.run([d_sc, d_sc[:777], d_sc[:1]]))
+    for i, k in enumerate((n, 777, 1)):
+        assert np.array_equal(got[i], O.msm(pts[:k], sc[:k]))
+    b.close()
+    ctx.close()

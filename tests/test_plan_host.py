@@ -14,9 +14,12 @@ PKG = os.path.join(HERE, "..", "impeller_b200")
 CUDA = os.path.dirname(os.path.dirname(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"))
 
 SOURCE = r"""
+#include <unistd.h>
+
 #include <cstdio>
 #include <cstring>
 #include "engine.h"
+#include "impeller_msm.h"
 using namespace impeller;
 
 // A context of len points as impeller_ctx_create makes it, without a device.
@@ -52,7 +55,41 @@ static int mixed_batch() {
     return 0;
 }
 
+static int largest() {
+    // sizes whose whole scalars' digits fit 32 bits and the halves' do not
+    Context k(280000000);
+    Plan p;
+    const u32 n = (u32)k.ctx.len, c = ctx_window(&k.ctx, n);
+    const bool one = Plan::build(p, 0, {ctx_shape(&k.ctx, n, c)});
+    std::printf("single %d %u\n", one, p.phi_points);
+    // the same of many MSMs together, through the call that makes a batch (it
+    // gets as far as the device)
+    if (!access("/dev/nvidiactl", F_OK)) {
+        std::printf("batch skipped\n");
+        return 0;
+    }
+    Context m(1 << 24);
+    std::vector<uint64_t> sizes(16, 1 << 24);
+    impeller_batch *b = nullptr;
+    const cudaError_t e = impeller_batch_create(&b, &m.ctx, sizes.data(), nullptr, (u32)sizes.size(), 0);
+    std::printf("batch %s\n", e == cudaErrorInvalidValue ? impeller_last_error() : "laid out");
+    return 0;
+}
+
+static int refused() {
+    // windows whose buckets do not fit are refused whether or not scalars are split
+    Context k(1 << 16);
+    for (u32 c : {28u, 29u, 30u, 31u}) {
+        Plan p;
+        const bool ok = Plan::build(p, 0, {ctx_shape(&k.ctx, 1000, c)});
+        std::printf("c%u %d\n", c, ok);
+    }
+    return 0;
+}
+
 int main(int argc, char **argv) {
+    if (argc > 1 && !std::strcmp(argv[1], "largest")) return largest();
+    if (argc > 1 && !std::strcmp(argv[1], "refused")) return refused();
     if (argc > 1 && !std::strcmp(argv[1], "mixed_batch")) return mixed_batch();
     return 2;
 }
@@ -70,7 +107,8 @@ def plans():
     src, exe = os.path.join(d, "plans.cpp"), os.path.join(d, "plans")
     with open(src, "w") as f:
         f.write(SOURCE)
-    subprocess.run([gxx, "-O1", "-std=c++17", "-I", os.path.join(PKG, "csrc"), "-I", os.path.join(CUDA, "include"), src,
+    subprocess.run([gxx, "-O1", "-std=c++17", "-I", os.path.join(PKG, "csrc"), "-I", os.path.join(HERE, "..", "include"),
+                    "-I", os.path.join(CUDA, "include"), src,
                     "-o", exe, build.LIB, "-Wl,-rpath," + os.path.abspath(PKG), "-lpthread"], check=True)
 
     def run(what):
@@ -86,3 +124,14 @@ def test_images_lie_past_every_point_of_a_batch(plans):
     assert r["built"] == "1 1 1"
     assert r["images_past_points"] == "1 1 1"
     assert r["images"] == "3000 3000 3000"
+
+
+def test_sizes_that_fit_with_whole_scalars_are_not_refused(plans):
+    r = plans("largest")
+    assert r["single"] == "1 0"
+    assert r["batch"] in ("laid out", "skipped")
+
+
+def test_windows_with_too_many_buckets_are_refused(plans):
+    # 2^31 buckets of whole scalars: from window 29 on (9 windows of 2^28)
+    assert plans("refused") == {"c28": "1", "c29": "0", "c30": "0", "c31": "0"}
