@@ -111,6 +111,7 @@ struct CardLayout {
     u64 card_off = 0, card_len = 0, part_len = 0;
     size_t o_points = 0, o_scalars = 0, o_carry = 0, o_results = 0, o_combine = 0, o_plan = 0, o_acc = 0;
     size_t o_images = 0, image_cap = 0, bytes = 0;  // streamed: one table image per chunk
+    size_t plan_bytes = 0;                          // scratch of any run's plan
 };
 
 // Chunk boundaries of a resident (parts == 1) range of `len` points that
@@ -151,7 +152,7 @@ std::vector<MsmShape> group_shapes(const Config &cfg, u32 M, u32 n, u32 part_len
 }
 
 bool card_layout(const Config &cfg, int device, u64 len, u32 num_cards, u32 card, u32 parts, u32 batch_per_run,
-                 CardLayout &L, size_t &plan_bytes) {
+                 CardLayout &L) {
     const u64 per_card = (len + num_cards - 1) / num_cards;
     L.card_off = std::min<u64>(len, (u64)card * per_card);
     L.card_len = std::min<u64>(per_card, len - L.card_off);
@@ -160,19 +161,22 @@ bool card_layout(const Config &cfg, int device, u64 len, u32 num_cards, u32 card
         set_error("part length times window tables exceeds 2^31 points; raise `parts`");
         return false;
     }
-    plan_bytes = 0;
-    size_t acc_bytes = 0, images = 0;
+    size_t plan_bytes = 0, acc_bytes = 0, images = 0;
     if (L.part_len) {
-        Plan p;
-        if (!Plan::build(p, device, group_shapes(cfg, batch_per_run, (u32)L.part_len, (u32)L.part_len))) return false;
-        plan_bytes = p.scratch_bytes();
+        const MsmShape shape = group_shapes(cfg, 1, (u32)L.part_len, (u32)L.part_len)[0];
+        RunSizes run;
+        if (!run_sizes(device, shape, batch_per_run, run)) return false;
+        plan_bytes = run.scratch;
         const u64 nchunks = parts > 1 ? (L.card_len + L.part_len - 1) / L.part_len : stream_chunks(L.card_len);
         if (nchunks > 1) {
+            Plan p;
+            if (!Plan::build(p, device, std::vector<MsmShape>(batch_per_run, shape))) return false;
             acc_bytes = p.acc_bytes();
-            L.image_cap = align_up(p.image_bytes(), 256);
+            L.image_cap = run.image;
             images = nchunks * L.image_cap;
         }
     }
+    L.plan_bytes = plan_bytes;
     const size_t stages = parts > 1 ? PART_STAGES : 1;
     size_t off = 0;
     auto take = [&](size_t b) {
@@ -264,9 +268,16 @@ DevicePlans &device_plans(int device) {
 
 constexpr size_t PLAN_CACHE_CAP = 32;
 
-Plan *cached_plan(DevicePlans &D, int device, const Config &cfg, u32 M, u32 n, u32 stride) {
+// A plan of at most `scratch` bytes.
+Plan *cached_plan(DevicePlans &D, int device, const Config &cfg, u32 M, u32 n, u32 stride, size_t scratch) {
     std::vector<u32> key{cfg.c, cfg.n_windows, M, n, stride, cfg.curve, cfg.glv ? 1u : 0u};
     auto it = D.plans.find(key);
+    if (it != D.plans.end() && it->second.plan->scratch_bytes() > scratch) {
+        // made for a call whose runs are larger (every plan of this call is within `scratch`)
+        D.plans.erase(it);
+        D.order.erase(std::find(D.order.begin(), D.order.end(), key));
+        it = D.plans.end();
+    }
     if (it != D.plans.end()) {
         it->second.gen = D.gen;
         return it->second.plan.get();
@@ -282,7 +293,7 @@ Plan *cached_plan(DevicePlans &D, int device, const Config &cfg, u32 M, u32 n, u
         }
     }
     std::unique_ptr<Plan> p(new Plan());
-    if (!Plan::build(*p, device, group_shapes(cfg, M, n, stride))) return nullptr;
+    if (!Plan::build_within(*p, device, group_shapes(cfg, M, n, stride), scratch)) return nullptr;
     Plan *raw = p.get();
     D.plans[key] = CachedPlan{std::move(p), D.gen};
     D.order.push_back(key);
@@ -358,7 +369,7 @@ cudaError_t run_card(CardJob &J) {
                                    cudaMemcpyHostToDevice, st));
                 sc[b] = dst;
             }
-            Plan *plan = cached_plan(D, J.device, cfg, M, (u32)card_len, stride);
+            Plan *plan = cached_plan(D, J.device, cfg, M, (u32)card_len, stride, J.L.plan_bytes);
             if (!plan) return cudaErrorInvalidValue;
             cudaError_t e = plan->enqueue(plan_scratch, d_points, sc.data(), d_results, mode, st, d_carry);
             if (e != cudaSuccess) return e;
@@ -387,7 +398,7 @@ cudaError_t run_card(CardJob &J) {
                 for (u32 b = 0; b < M; b++)
                     sc[b] = staged ? d_scalars + slot * scalar_stage + (size_t)b * part_len * 8
                                    : d_scalars + (size_t)b * part_len * 8 + s0 * 8;
-                chunk_plan[k] = cached_plan(D, J.device, cfg, M, (u32)mk, stride);
+                chunk_plan[k] = cached_plan(D, J.device, cfg, M, (u32)mk, stride, J.L.plan_bytes);
                 if (!chunk_plan[k]) return cudaErrorInvalidValue;
                 if (chunk_plan[k]->image_bytes() > J.L.image_cap) {
                     set_error("msm: chunk table image exceeds its slot");
@@ -535,8 +546,7 @@ cudaError_t impeller_msm_cfg_curve(unsigned int curve, unsigned int window_size,
     }
     std::vector<CardLayout> layouts(num_cards);
     for (u32 i = 0; i < num_cards; i++) {
-        size_t pb = 0;
-        if (!card_layout(cfg, (int)cards[i], len, num_cards, i, parts, batch_per_run, layouts[i], pb))
+        if (!card_layout(cfg, (int)cards[i], len, num_cards, i, parts, batch_per_run, layouts[i]))
             return cudaErrorInvalidValue;
     }
     if (buffers == nullptr) {

@@ -226,7 +226,8 @@ static u32 pair_level_count(u64 entries, u64 nb, int sms, u32 curve) {
     return pair_levels(entries, nb, pair_slots_min(sms, curve), PAIR_MAX_LEVELS);
 }
 
-bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool resident, bool no_pairs) {
+bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool resident, bool no_pairs,
+                 bool entry_sort) {
     p.device = device;
     p.shapes = shapes;
     p.M = (u32)shapes.size();
@@ -426,7 +427,7 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
         bin_cell[nbins] = (u32)std::min<u64>(cells, 0xffffffffu);
     }
     p.small_sort = resident && p.M == 1 && entries <= SMALL_SORT_ENTRIES && nb <= SMALL_SORT_BUCKETS;
-    p.msd = !p.small_sort && stiles > 0 && nbins <= SORT_MAX_BINS && cells <= SORT_MAX_CELLS;
+    p.msd = !p.small_sort && !entry_sort && stiles > 0 && nbins <= SORT_MAX_BINS && cells <= SORT_MAX_CELLS;
     if (p.msd) {
         p.nbins = (u32)nbins;
         p.sort_tiles = (u32)stiles;
@@ -497,6 +498,49 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
     lo.o_carry = take((size_t)p.M * XB);
     lo.o_results = take((size_t)p.M * PB);
     lo.bytes = off;
+    return true;
+}
+
+bool Plan::build_within(Plan &p, int device, const std::vector<MsmShape> &shapes, size_t scratch) {
+    if (!build(p, device, shapes)) return false;
+    if (p.scratch_bytes() <= scratch) return true;
+    if (!build(p, device, shapes, false, false, true)) return false;
+    if (p.scratch_bytes() <= scratch) return true;
+    set_error("plan exceeds its scratch");
+    return false;
+}
+
+bool run_sizes(int device, const MsmShape &shape, u32 msms, RunSizes &out) {
+    // kept by the sizes: a call with many MSMs a run would lay them all out again
+    typedef std::vector<u32> Key;
+    static std::mutex mu;
+    static std::map<Key, RunSizes> known;
+    constexpr size_t KNOWN_MAX = 256;
+    const Key key{shape.n, shape.c, shape.n_windows, shape.table_stride, shape.table_base, shape.curve,
+                  shape.split ? 1u : 0u, msms, (u32)sm_count(device)};
+    {
+        std::lock_guard<std::mutex> g(mu);
+        auto it = known.find(key);
+        if (it != known.end()) {
+            out = it->second;
+            return true;
+        }
+    }
+    out = RunSizes{};
+    // every number of MSMs up to 64, then one in so many (a plan between them
+    // that needed more would be refused by build_within)
+    const u32 step = (msms + 63) / 64;
+    for (u32 k = msms; k; k = k > step ? k - step : 0) {
+        Plan p;
+        if (!Plan::build(p, device, std::vector<MsmShape>(k, shape))) return false;
+        out.scratch = std::max(out.scratch, p.scratch_bytes());
+        // (fewer points may take the two-level sort, whose image lists its bins)
+        const size_t bins = p.msd ? 0 : align_up((size_t)(p.nb / FINE + 2) * 4, 16);
+        out.image = std::max(out.image, align_up(p.image_bytes() + bins, 256));
+    }
+    std::lock_guard<std::mutex> g(mu);
+    if (known.size() >= KNOWN_MAX) known.clear();
+    known[key] = out;
     return true;
 }
 

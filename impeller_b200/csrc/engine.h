@@ -73,8 +73,12 @@ class Plan {
     // (no_pairs: not; the levels' points take scratch), and a single small MSM
     // takes the one-block sort.  Plans built for a footprint (the server's,
     // the drop-in call's) keep the layout whose sizes add up over jobs.
+    // entry_sort: the per-entry sort, in less scratch, where the two-level one
+    // would be taken.
     static bool build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool resident = false,
-                      bool no_pairs = false);
+                      bool no_pairs = false, bool entry_sort = false);
+    // A plan within `scratch` bytes, with the per-entry sort where it takes that.
+    static bool build_within(Plan &p, int device, const std::vector<MsmShape> &shapes, size_t scratch);
     // Whether a plan of these shapes would sort its entries with the
     // two-level counting sort (fast) rather than the per-entry atomic sort
     // that build() falls back to for very large batches.
@@ -198,6 +202,15 @@ class Plan {
     u32 prof_used = 0;
     cudaError_t prof_mark(int k, cudaStream_t st);
 };
+
+// What any run of 1 to `msms` MSMs of a shape needs: scratch, and its table image.
+// More MSMs may need less: past its limits the sort takes less scratch, and the
+// bucket reduction's chunks double.  A run of fewer points than the shape's fits
+// too, built by Plan::build_within.
+struct RunSizes {
+    size_t scratch = 0, image = 0;
+};
+bool run_sizes(int device, const MsmShape &shape, u32 msms, RunSizes &out);
 
 // Scratch from a per-device pool (engine.cu): stream-ordered like
 // cudaMallocAsync, freed with cudaFreeAsync.  Holders keep freed scratch mapped.

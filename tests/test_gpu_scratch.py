@@ -102,3 +102,20 @@ def test_whole_scalars_where_the_images_find_no_room(M):
         assert np.array_equal(got[i], O.msm(pts[:k], sc[:k]))
     b.close()
     ctx.close()
+
+
+def test_last_run_of_a_drop_in_call_with_fewer_msms(M):
+    # five MSMs a run sort entry by entry, the four that there are in two
+    # levels, which takes more scratch: all within the buffer
+    n, guard = 1_000_000, 1 << 20
+    op = M.MSM(M.MsmConfig(window_size=18, target_window=15, batch_per_run=5))
+    size = op.get_buffer_size(n)[0]
+    buf, keep = M.alloc_gpu_buffer(size + guard)
+    keep[size:] = 0xA5
+    pts = M.to_host(M.gen_points_device(n, seed=24)).reshape(n, -1)
+    sc = [M.to_host(M.gen_scalars_device(n, seed=24, stream_id=i)).reshape(n, 8) for i in (1, 2)]
+    got = op.run([pts], [sc[0], sc[1], sc[1], sc[0]], [buf])
+    assert bool((keep[size:] == 0xA5).all())
+    want = [O.msm(pts, s) for s in sc]
+    for g, k in zip(got, (0, 1, 1, 0)):
+        assert np.array_equal(g, want[k])

@@ -87,7 +87,40 @@ static int refused() {
     return 0;
 }
 
+static int runs() {
+    // a drop-in call sizes its buffer for its largest run; the last run has
+    // fewer MSMs, and a streamed one fewer points
+    u32 checked = 0, larger = 0, refused = 0, over = 0;
+    for (u32 curve : {(u32)CURVE_BN254, (u32)CURVE_BLS12381})
+        for (u32 c : {4u, 8u, 11u, 12u, 14u, 16u, 18u, 19u, 20u, 22u})
+            for (u32 kind = 0; kind < 3; kind++)
+                for (u32 n : {1u, 300u, 5000u, 100003u, 1000000u, 1u << 21})
+                    for (u32 msms : {2u, 3u, 5u, 7u, 16u, 64u}) {
+                        if ((u64)n * msms > 8000000) continue;
+                        MsmShape s{n, c, kind == 0 ? 0 : kind == 1 ? 4u : 1u, n, 0, curve};
+                        if (kind == 0) s.split = curve == CURVE_BN254;
+                        RunSizes r;
+                        Plan full;
+                        if (!Plan::build(full, 0, std::vector<MsmShape>(msms, s)) || !run_sizes(0, s, msms, r)) continue;
+                        for (u32 k = 1; k <= msms; k = k < 8 ? k + 1 : k * 5 / 4)
+                            for (u32 m : {n, n - n / 10, n / 3 + 1, 1u}) {
+                                Plan p;
+                                MsmShape t = s;
+                                t.n = m;
+                                checked++;
+                                if (!Plan::build_within(p, 0, std::vector<MsmShape>(k, t), r.scratch)) refused++;
+                                else if (p.scratch_bytes() > r.scratch || p.image_bytes() > r.image) over++;
+                                Plan q;
+                                Plan::build(q, 0, std::vector<MsmShape>(k, t));
+                                larger += q.scratch_bytes() > full.scratch_bytes() || q.image_bytes() > full.image_bytes();
+                            }
+                    }
+    std::printf("checked %u\nlarger %u\nrefused %u\nover %u\n", checked, larger, refused, over);
+    return 0;
+}
+
 int main(int argc, char **argv) {
+    if (argc > 1 && !std::strcmp(argv[1], "runs")) return runs();
     if (argc > 1 && !std::strcmp(argv[1], "largest")) return largest();
     if (argc > 1 && !std::strcmp(argv[1], "refused")) return refused();
     if (argc > 1 && !std::strcmp(argv[1], "mixed_batch")) return mixed_batch();
@@ -135,3 +168,10 @@ def test_sizes_that_fit_with_whole_scalars_are_not_refused(plans):
 def test_windows_with_too_many_buckets_are_refused(plans):
     # 2^31 buckets of whole scalars: from window 29 on (9 windows of 2^28)
     assert plans("refused") == {"c28": "1", "c29": "0", "c30": "0", "c31": "0"}
+
+
+def test_every_run_of_a_drop_in_call_fits_its_buffer(plans):
+    r = plans("runs")
+    assert int(r["checked"]) > 5000
+    assert int(r["larger"]) > 0  # smaller runs that need more than the largest: the case in question
+    assert r["refused"] == "0" and r["over"] == "0"
