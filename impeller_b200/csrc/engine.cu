@@ -91,7 +91,9 @@ int sm_count(int device) {
 // Scratch memory that outlives one context: freed scratch stays mapped for the
 // next context or batch, so that a new one's first MSM does not wait for the
 // mapping (4 to 5 ms per GB).  At most SCRATCH_KEEP bytes per device stay,
-// and none once the device's last holder is gone.
+// and none once the device's last holder is gone.  cudaMalloc takes what is
+// freed here when the device has no other memory left, but cudaMemGetInfo
+// counts it as used: scratch_trim gives it back.
 static constexpr u64 SCRATCH_KEEP = 6ull << 30;
 
 struct ScratchPool {
@@ -124,6 +126,14 @@ void scratch_release(int device) {
         cudaStreamSynchronize(nullptr);  // the frees before this
         cudaMemPoolTrimTo(p.pool, 0);
     }
+}
+
+void scratch_trim(int device) {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    auto it = g_pools.find(device);
+    if (it == g_pools.end() || !it->second.pool) return;
+    cudaDeviceSynchronize();  // frees that are still in a stream
+    cudaMemPoolTrimTo(it->second.pool, 0);
 }
 
 // Test hook: the next of these steps fails (0: none).

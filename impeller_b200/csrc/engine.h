@@ -216,6 +216,7 @@ bool run_sizes(int device, const MsmShape &shape, u32 msms, RunSizes &out);
 // cudaMallocAsync, freed with cudaFreeAsync.  Holders keep freed scratch mapped.
 cudaError_t scratch_hold(int device);
 void scratch_release(int device);
+void scratch_trim(int device);  // the current device: gives freed scratch back to the system
 cudaError_t scratch_alloc(void **out, size_t bytes, int device, cudaStream_t st);
 
 // k_combine: sum `k` XYZZ points in device memory, write canonical affine.

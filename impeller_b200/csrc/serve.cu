@@ -352,6 +352,7 @@ cudaError_t impeller_server_create(impeller_server **out, impeller_ctx *ctx, uin
     s->max_inflight = max_inflight;
     cudaError_t e = setup_step("cudaSetDevice", cudaSetDevice(ctx->device));
     if (e != cudaSuccess) return e;
+    scratch_trim(ctx->device);  // contexts' freed scratch is the server's to use
     if (hbm_budget == 0) {
         size_t fr = 0, tot = 0;
         if ((e = setup_step("cudaMemGetInfo", cudaMemGetInfo(&fr, &tot))) != cudaSuccess) return e;

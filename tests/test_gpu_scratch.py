@@ -119,3 +119,23 @@ def test_last_run_of_a_drop_in_call_with_fewer_msms(M):
     want = [O.msm(pts, s) for s in sc]
     for g, k in zip(got, (0, 1, 1, 0)):
         assert np.array_equal(g, want[k])
+
+
+def test_server_budget_counts_freed_scratch(M):
+    # scratch that a closed context left in the pool is free for a server
+    n = 1 << 21
+    keep = M.MsmContext(O.gen_points(100, seed=25))  # the pool lives
+    ctx = M.MsmContext(M.gen_points_device(n, seed=25))
+    sc = M.gen_scalars_device(n, seed=25)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    ctx.msm_device(sc)
+    torch.cuda.synchronize()
+    used = free - torch.cuda.mem_get_info()[0]
+    assert used > 1 << 28
+    ctx.close()
+    srv = M.MsmServer(keep, max_batch=2, max_inflight=1)
+    budget = srv.stats()["budget_bytes"]
+    srv.close()
+    keep.close()
+    assert budget > free - (1 << 30) - used // 4
