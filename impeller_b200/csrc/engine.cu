@@ -128,6 +128,18 @@ void scratch_release(int device) {
     }
 }
 
+// Bytes that the pool holds and nobody uses.
+static size_t scratch_idle(int device) {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    auto it = g_pools.find(device);
+    u64 held = 0, used = 0;
+    if (it == g_pools.end() || !it->second.pool ||
+        cudaMemPoolGetAttribute(it->second.pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+        cudaMemPoolGetAttribute(it->second.pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess || used > held)
+        return 0;
+    return (size_t)(held - used);
+}
+
 void scratch_trim(int device) {
     std::lock_guard<std::mutex> g(g_pool_mu);
     auto it = g_pools.find(device);
@@ -1226,6 +1238,20 @@ static Plan *ctx_plan(impeller_ctx *ctx, u32 n, u32 c, PlanKind kind = PLAN_FULL
     return raw;
 }
 
+// Whether the affine levels of a plan leave the device most of its memory: they
+// take three quarters of a point per digit (3 GB at 2^22 points with tables, up
+// to 25 GB) for a tenth of the time, so never more than a quarter of what is
+// free, `had` bytes that the plan's scratch replaces included.
+static bool levels_leave_room(const Plan &p, size_t had) {
+    if (!p.pair_levels || p.scratch_bytes() <= had) return true;
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return true;
+    }
+    return p.layout.o_phi - p.layout.o_pair_odd <= (free_bytes + scratch_idle(p.device) + had) / 4;
+}
+
 extern "C" {
 
 const char *impeller_last_error(void) { return impeller::last_error(); }
@@ -1384,7 +1410,7 @@ static cudaError_t ctx_run_locked(impeller_ctx *ctx, const uint32_t *d_scalars, 
     Plan *p = ctx_plan(ctx, (u32)n, c);
     if (!p) return cudaErrorInvalidValue;
     const size_t had = ctx->scratch_bytes;
-    cudaError_t e = ctx_reserve(ctx, p->scratch_bytes(), stream);
+    cudaError_t e = levels_leave_room(*p, had) ? ctx_reserve(ctx, p->scratch_bytes(), stream) : cudaErrorMemoryAllocation;
     while (e == cudaErrorMemoryAllocation && (p->pair_levels || p->phi_points)) {
         // no room for the affine levels' points, then none for the images: the
         // plan without them, in no less scratch than there was, so that other
@@ -1530,7 +1556,9 @@ cudaError_t impeller_batch_create(impeller_batch **out, impeller_ctx *ctx, const
     CK(cudaSetDevice(ctx->device));
     CK(scratch_hold(ctx->device));
     b->held = true;
-    cudaError_t e = scratch_alloc(&b->scratch, b->plan.scratch_bytes(), ctx->device, nullptr);
+    cudaError_t e = levels_leave_room(b->plan, 0)
+                        ? scratch_alloc(&b->scratch, b->plan.scratch_bytes(), ctx->device, nullptr)
+                        : cudaErrorMemoryAllocation;
     while (e == cudaErrorMemoryAllocation && (b->plan.pair_levels || b->plan.phi_points)) {
         // no room for the affine levels' points, then none for the images
         (void)cudaGetLastError();

@@ -69,6 +69,31 @@ def test_plan_without_levels_takes_over_until_the_scratch_grows(M, leveled):
     ctx.close()
 
 
+def test_levels_take_a_quarter_of_the_free_memory_at_most(M, leveled):
+    pts, sc, want, small, want_small = leveled
+    ctx, room = M.MsmContext(pts), M.MsmContext(pts)
+    full = room.launches(N, C)
+    # the levels take 0.75 points of 64 bytes a digit: 0.8 GB
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - (5 << 29), dtype=torch.uint8, device="cuda")
+    d_sc = M.to_device(sc)
+    assert np.array_equal(M.to_host(ctx.msm_device(d_sc, c=C)), want)
+    assert ctx.launches(N, C) < full
+    b = ctx.batch([N, 900], windows=[C, 8], graph=False)
+    got = M.to_host(b.run([d_sc, M.to_device(small)]))
+    assert np.array_equal(got[0], want) and np.array_equal(got[1], want_small)
+    less = b.launches
+    b.close()
+    del hold
+    torch.cuda.empty_cache()
+    b = ctx.batch([N, 900], windows=[C, 8], graph=False)
+    assert b.launches > less
+    b.close()
+    assert np.array_equal(M.to_host(room.msm_device(d_sc, c=C)), want)
+    assert room.launches(N, C) == full
+    room.close()
+    ctx.close()
+
+
 def test_batch_without_room_for_levels(M, leveled):
     pts, sc, want, small, want_small = leveled
     ctx = M.MsmContext(pts)
