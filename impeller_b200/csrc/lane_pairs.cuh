@@ -42,9 +42,23 @@ __device__ __noinline__ XyzzT<F> xyzz_dbl_call(XyzzT<F> p) {
     return xyzz_dbl<F, MulCall>(p);
 }
 
-// add-2008-s; every special case.
+// Whether zz can be zero, from its low word.
+template <class F>
+__device__ __forceinline__ bool pair_maybe_identity(const XyzzT<F> &p) {
+    constexpr Words<F::N> m = words(F::M);
+    return p.zz.l[0] == 0 || p.zz.l[0] == m.v[0];
+}
+
+// add-2008-s; every special case.  Empty buckets are common (a zero polynomial;
+// a column of small values leaves all windows but the lowest empty), so lanes
+// that all add the identity leave early: 2^10 to 2^20 zero scalars on plain
+// windows 0.40 to 0.51 ms without, 0.08 to 0.17 with.
 template <class F>
 __device__ __forceinline__ XyzzT<F> xyzz_add_pair(const XyzzT<F> &p, const XyzzT<F> &q, bool odd, u32 mask) {
+    if (__all_sync(mask, pair_maybe_identity(p) || pair_maybe_identity(q))) {
+        const bool id = xyzz_is_identity(p);
+        if (__all_sync(mask, id || xyzz_is_identity(q))) return id ? q : p;
+    }
     const Fe<F> u = fe_mul(fe_pick(odd, p.x, q.x), fe_pick(odd, q.zz, p.zz));    // u1 | u2
     const Fe<F> s = fe_mul(fe_pick(odd, p.y, q.y), fe_pick(odd, q.zzz, p.zzz));  // s1 | s2
     // P and R in the even lane, their negatives in the odd one
@@ -93,7 +107,7 @@ __device__ __forceinline__ JacT<F> jac_dbl_pair(const JacT<F> &p, bool odd, u32 
 // 2^k p through Jacobian coordinates (xyzz_dbl_n); the identity stays so.
 template <class F>
 __device__ __forceinline__ XyzzT<F> xyzz_dbl_n_pair(const XyzzT<F> &p, u32 k, bool odd, u32 mask) {
-    if (k == 0) return p;
+    if (k == 0 || __all_sync(mask, xyzz_is_identity(p))) return p;
     JacT<F> j;
     j.x = fe_mul(p.x, fe_sqr(p.zz));
     j.y = fe_mul(p.y, fe_sqr(p.zzz));
