@@ -432,10 +432,11 @@ struct PassPlan {
 
 // Tile of a transform of more than 2^11 elements.
 //
-// Up to 2^20 elements two passes of half of the index bits each: the data lie
-// in L2, so that short runs cost little, and small tiles spread a small
-// transform over the SMs (2^12: 36 -> 20 us against a tile of 2^10, 2^16:
-// 51 -> 37, 2^20: 237 -> 219 against 9 and 11 bits).
+// Up to 2^20 elements two passes of about half of the index bits each: the data
+// lie in L2, so that short runs cost little, and small tiles spread a small
+// transform over the SMs (2^12: 36 -> 20 us against a tile of 2^10; 2^16: 51 ->
+// 35 against 2^11).  From 2^18 on tiles of 2^10, whose runs are whole sectors
+// and more (2^18: 72 us, 73 with tiles of 2^9, 82 with 2^11).
 //
 // Above, tiles of 2^10 elements (128 threads, six blocks per SM) keep the
 // multipliers busier than tiles of 2^11 (three of 256 threads), as more blocks
@@ -443,7 +444,7 @@ struct PassPlan {
 // nor cut the global runs below 256 bytes.  2^24 elements: 3.74 ms with tiles
 // of 2^11, 3.47 with 2^10.
 u32 tile_log(u32 L) {
-    if (L <= 2 * (TILE_LOG - 1)) return L <= 16 ? 8 : (L + 1) / 2;
+    if (L <= 2 * (TILE_LOG - 1)) return L <= 16 ? 8 : L == 17 ? 9 : TILE_LOG - 1;
     const u32 np = (L - TILE_LOG + MID_MAX - 1) / MID_MAX, np_small = (L - (TILE_LOG - 1) + MID_MAX - 1) / MID_MAX;
     const u32 digit = (L - (TILE_LOG - 1) + np_small - 1) / np_small;
     return np_small == np && digit + 3 <= TILE_LOG - 1 ? TILE_LOG - 1 : TILE_LOG;
@@ -475,15 +476,24 @@ cudaError_t run_ntt(const View &v, const u32 *tw, u32 L, cudaStream_t st) {
     }
     auto kern = k_ntt_pass<F, RECOMP>;
     NTT_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE * 32));
+    // 256 blocks leave room beside them on every SM.  Where those of the next
+    // pass are set up ahead they take it unevenly, three on some SMs and none on
+    // others, and the pass lasts as long as the fullest one (2^18: 87 us with
+    // chained launches, 72 with plain ones; 2^16: 37 and 35).
+    const bool chain = L < 16 || L > 18;
     for (const PassPlan &pp : plan_passes(L)) {
         const u32 tile = pp.R + pp.logC;
-        // up to 2^17 elements a thread takes one quad of elements a round
-        // instead of two: there are SMs to spare
-        impeller::launch_next(kern, (unsigned)(1ull << (L - tile)), 1u << (tile - (L <= 17 ? 2 : 3)), (size_t)32 << tile, st, v, tw, L,
-                              pp.lo, pp.R, pp.logC);
+        // up to 2^20 elements a thread takes one quad of elements a round instead
+        // of two: there are SMs to spare (2^19: 161 -> 119 us, 2^20: 228 -> 211)
+        const u32 threads = 1u << (tile - (L <= 20 ? 2 : 3)), blocks = (u32)(1ull << (L - tile));
+        const size_t smem = (size_t)32 << tile;
+        if (chain) impeller::launch_next(kern, blocks, threads, smem, st, v, tw, L, pp.lo, pp.R, pp.logC);
+        else kern<<<blocks, threads, smem, st>>>(v, tw, L, pp.lo, pp.R, pp.logC);
         NTT_CK(launched("k_ntt_pass"));
     }
-    impeller::launch_next(k_ntt_reverse<F>, 1u << (L - 2 * REV_T), 256, 0, st, v, L);
+    const u32 blocks = 1u << (L - 2 * REV_T);
+    if (chain) impeller::launch_next(k_ntt_reverse<F>, blocks, 256, 0, st, v, L);
+    else k_ntt_reverse<F><<<blocks, 256, 0, st>>>(v, L);
     return launched("k_ntt_reverse");
 }
 
