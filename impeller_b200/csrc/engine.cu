@@ -1386,10 +1386,16 @@ cudaError_t impeller_ctx_precompute(impeller_ctx *ctx, unsigned int c) {
         set_error(std::string("impeller_ctx_precompute: ") + cudaGetErrorString(e));
         return e;
     }
-    if (ctx->tables) cudaFree(ctx->tables);
-    ctx->tables = t;
-    ctx->tables_points = total;
-    ctx->sets.emplace_back(c, (u32)have);
+    {
+        std::unique_lock<std::shared_mutex> change(ctx->tables_mu);
+        if (ctx->tables) {
+            cudaDeviceSynchronize();  // batches launched on them meanwhile
+            cudaFree(ctx->tables);
+        }
+        ctx->tables = t;
+        ctx->tables_points = total;
+        ctx->sets.emplace_back(c, (u32)have);
+    }
     ctx->plans.clear();
     return cudaSuccess;
 }

@@ -8,6 +8,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <shared_mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -248,6 +249,10 @@ struct impeller_ctx {
     // Resident window tables: one allocation holding the points (region 0)
     // followed by table sets; the set for window c has W(c) tables of len
     // points, table j = 2^(j*c) * P, starting at point index base.
+    // They change under mu and tables_mu; those who read them without mu (the
+    // server, whose jobs are submitted while batches are launched) share
+    // tables_mu until what they launch on them is in its stream.
+    std::shared_mutex tables_mu;
     impeller::u32 *tables = nullptr;
     impeller::u64 tables_points = 0;  // points held by `tables`
     std::vector<std::pair<impeller::u32, impeller::u32>> sets;  // (c, base)

@@ -134,7 +134,7 @@ cudaError_t launch_batch(impeller_server *s, Batch &b, std::vector<Job *> &js, u
     {
         // a table build in another thread frees the previous tables, after
         // waiting for what has been launched on them
-        std::lock_guard<std::mutex> g(s->ctx->mu);
+        std::shared_lock<std::shared_mutex> g(s->ctx->tables_mu);
         e = b.plan->enqueue(base + o_plan, ctx_point_base(s->ctx), sc.data(), d_res, 0, b.stream);
     }
     if (e != cudaSuccess) return e;
@@ -384,7 +384,7 @@ cudaError_t impeller_server_submit(impeller_server *s, const uint32_t *h_scalars
     // whole scalars where the split ones' images do not fit the budget
     for (const bool whole : {false, true}) {
         {
-            std::lock_guard<std::mutex> g(s->ctx->mu);  // the table sets may be growing
+            std::shared_lock<std::shared_mutex> g(s->ctx->tables_mu);  // the table sets may be growing
             j.c = ctx_window(s->ctx, n, whole);
             j.shape = ctx_shape(s->ctx, (u32)n, j.c, whole);
         }
