@@ -889,10 +889,8 @@ cudaError_t Plan::run_tail(void *scratch, const u32 *buckets, bool dense, u32 *r
     const PlanPtrs p = plan_ptrs(layout, desc_off, win_off, blk_off, tf_off, scratch, carry_ext, results, d_image);
     cudaError_t pe;
     ReduceArgs ra{p.wins, p.blk, pair_levels ? p.level_offsets : p.offsets, buckets, p.parts, p.parts_s, dense ? 1u : 0u};
-    // k_reduce's blocks fill half of the chip: set up ahead they crowd onto the
-    // SMs that the fixups leave first (2^20 skewed: 1.92 ms against 1.87).
     if (reduce_pairs) CURVE_LAUNCH(curve, k_reduce_pairs, nrblocks, REDUCE_BLOCK, 0, st, ra);
-    else CURVE_LAUNCH_PLAIN(curve, k_reduce, nrblocks, REDUCE_BLOCK, 0, st, ra);
+    else CURVE_LAUNCH(curve, k_reduce, nrblocks, REDUCE_BLOCK, 0, st, ra);
     CK_LAUNCH("k_reduce");
     MARK(7);
 

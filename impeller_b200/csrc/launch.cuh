@@ -2,16 +2,23 @@
 //
 // A chain of kernels of a few microseconds each pays for every hand-over: the
 // next kernel is only set up once the previous one has drained.  launch_next
-// lets it be set up beside the previous kernel (programmatic stream
-// serialization); grid_wait, the first thing such a kernel does, waits until
-// the previous kernel has completed and its writes are visible.  That orders
-// ordinary accesses as a plain launch does.  It does not order loads through
-// the read-only path (__ldg, or const __restrict__ parameters): the compiler
-// may take those ahead of the wait, and the hardware wants their data unwritten
-// from the kernel's start, which now lies before the previous kernel's end.  So
-// such a kernel reads with plain loads whatever a kernel of the chain writes;
-// only inputs that none of them writes (descriptors, the point array) may be
-// const __restrict__.
+// lets it be set up as soon as the previous kernel's blocks have ended
+// (programmatic stream serialization); grid_wait, the first thing such a kernel
+// does, waits until the previous kernel has completed and its writes are
+// visible.  That orders ordinary accesses as a plain launch does.  It does not
+// order loads through the read-only path (__ldg, or const __restrict__
+// parameters): the compiler may take those ahead of the wait, and the hardware
+// wants their data unwritten from the kernel's start, which now lies before the
+// previous kernel's end.  So such a kernel reads with plain loads whatever a
+// kernel of the chain writes; only inputs that none of them writes
+// (descriptors, the point array) may be const __restrict__.
+//
+// No kernel asks for its successor earlier (griddepcontrol.launch_dependents).
+// Blocks that are set up while others still run hold registers and shared
+// memory that other streams' kernels could use, and crowd onto the SMs that
+// have room.  With that request at the start of every kernel, three streams of
+// 10^5-point BLS12-381 MSMs took 1183 us an MSM (953 without), a transform of
+// 2^18 elements 87 us (65) and a lone MSM of 300 points 216 us (210).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -19,7 +26,7 @@
 namespace impeller {
 
 __device__ __forceinline__ void grid_wait() {
-    asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // kern<<<grid, block, smem, st>>>(args...) for a kernel that starts with grid_wait.

@@ -476,24 +476,15 @@ cudaError_t run_ntt(const View &v, const u32 *tw, u32 L, cudaStream_t st) {
     }
     auto kern = k_ntt_pass<F, RECOMP>;
     NTT_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE * 32));
-    // 256 blocks leave room beside them on every SM.  Where those of the next
-    // pass are set up ahead they take it unevenly, three on some SMs and none on
-    // others, and the pass lasts as long as the fullest one (2^18: 87 us with
-    // chained launches, 72 with plain ones; 2^16: 37 and 35).
-    const bool chain = L < 16 || L > 18;
     for (const PassPlan &pp : plan_passes(L)) {
         const u32 tile = pp.R + pp.logC;
         // up to 2^20 elements a thread takes one quad of elements a round instead
         // of two: there are SMs to spare (2^19: 161 -> 119 us, 2^20: 228 -> 211)
-        const u32 threads = 1u << (tile - (L <= 20 ? 2 : 3)), blocks = (u32)(1ull << (L - tile));
-        const size_t smem = (size_t)32 << tile;
-        if (chain) impeller::launch_next(kern, blocks, threads, smem, st, v, tw, L, pp.lo, pp.R, pp.logC);
-        else kern<<<blocks, threads, smem, st>>>(v, tw, L, pp.lo, pp.R, pp.logC);
+        impeller::launch_next(kern, (unsigned)(1ull << (L - tile)), 1u << (tile - (L <= 20 ? 2 : 3)), (size_t)32 << tile, st, v, tw, L,
+                              pp.lo, pp.R, pp.logC);
         NTT_CK(launched("k_ntt_pass"));
     }
-    const u32 blocks = 1u << (L - 2 * REV_T);
-    if (chain) impeller::launch_next(k_ntt_reverse<F>, blocks, 256, 0, st, v, L);
-    else k_ntt_reverse<F><<<blocks, 256, 0, st>>>(v, L);
+    impeller::launch_next(k_ntt_reverse<F>, 1u << (L - 2 * REV_T), 256, 0, st, v, L);
     return launched("k_ntt_reverse");
 }
 
