@@ -342,7 +342,7 @@ bool Plan::build(Plan &p, int device, const std::vector<MsmShape> &shapes, bool 
     // addition, half the additions at once): L leaves each warp a scheduler of
     // its own.
     p.reduce_pairs = nb <= REDUCE_PAIRS_MAX;
-        const u64 target = p.reduce_pairs ? (u64)sms * 64 : (u64)sms * REDUCE_LANES_PER_SM;
+    const u64 target = p.reduce_pairs ? (u64)sms * 64 : (u64)sms * REDUCE_LANES_PER_SM;
     u32 L = 1;
     while (nb / L > target && L < (1u << 30)) L <<= 1;
     std::vector<uint2> rblocks;
@@ -1222,6 +1222,7 @@ static Plan *ctx_plan(impeller_ctx *ctx, u32 n, u32 c, PlanKind kind = PLAN_FULL
     // A plan that took the place of one there was no room for holds until the
     // scratch is resized again (which waited for its last run).
     if (it != ctx->plans.end() && it->second->reduced_at && it->second->reduced_at != ctx->resizes) {
+        cudaSetDevice(ctx->device);  // its table image is freed there
         ctx->plans.erase(it);
         it = ctx->plans.end();
     }
