@@ -1,4 +1,4 @@
-// Pippenger MSM kernels for BN254 G1 on sm_100a.
+// Pippenger MSM kernels for BN254 and BLS12-381 G1 on sm_100a.
 //
 // One pass over a batch of M MSMs that share one device-resident point array:
 //

@@ -515,7 +515,8 @@ cudaError_t ntt_impl(PolyPtr x, const u32 *tw, u32 L, cudaStream_t st) {
 // Stream-ordered memory for the power tables of a recomputing transform.  The
 // device's default pool gives its memory back to the system whenever the
 // stream is waited for, and mapping it again cost 0.45 ms of a 0.5 ms call;
-// this pool keeps up to POOL_KEEP bytes (the pool maps 32 MB at a time) per device.
+// this pool keeps up to POOL_KEEP bytes (the pool maps 32 MB at a time) per
+// device, which cudaMalloc takes when the device is full.
 // A stream in capture takes the default route: its graph owns the memory.
 constexpr u64 POOL_KEEP = 64ull << 20;
 

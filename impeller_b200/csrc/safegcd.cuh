@@ -5,8 +5,10 @@
 // points), so variable time is fine.
 //
 // The method (D. J. Bernstein and B.-Y. Yang, "Fast constant-time gcd
-// computation and modular inversion", 2019, in the form that starts at
-// delta = 1/2) keeps an odd f (initially the modulus p), a g (initially the
+// computation and modular inversion", 2019; the form that starts at
+// delta = 1/2 is P. Wuille's, 2021, and this way of batching the steps is that
+// of the description of libsecp256k1's modular inversion by P. Dettman and
+// P. Wuille) keeps an odd f (initially the modulus p), a g (initially the
 // input x) and zeta = -(delta + 1/2), and applies divsteps: with g odd and
 // zeta < 0, (f, g) <- (g, (g - f) / 2) and zeta <- -zeta - 2; with g odd and
 // zeta >= 0, g <- (g + f) / 2 and zeta <- zeta - 1; with g even, g <- g / 2

@@ -7,7 +7,8 @@
  * Montgomery form (R = 2^256); an affine point is 16 uint32 (x then y),
  * byte-identical to halo2curves' G1Affine; the identity point is (0, 0).
  * Scalars are Fr elements in Montgomery form.  Results are canonical affine
- * points in the same form.
+ * points in the same form.  Points have to lie on the curve (without window
+ * tables BN254 scalars are split by its endomorphism).
  *
  * Return values are cudaError_t codes; argument errors return
  * cudaErrorInvalidValue and impeller_last_error() says why.
