@@ -88,6 +88,23 @@ int sm_count(int device) {
     return v;
 }
 
+// A device cannot be waited for while a stream of it captures a graph: the wait
+// fails and so does the capture.  Threads of this library take turns.
+static std::mutex g_capture_mu;
+
+static cudaError_t device_sync() {
+    std::lock_guard<std::mutex> g(g_capture_mu);
+    return cudaDeviceSynchronize();
+}
+
+// Waits for the device, or where that fails as a caller's thread captures on
+// it, for the event of the last run that used what is about to be freed.
+static void wait_idle(cudaEvent_t last_run) {
+    if (device_sync() == cudaSuccess) return;
+    (void)cudaGetLastError();
+    if (last_run) cudaEventSynchronize(last_run);
+}
+
 // Scratch memory that outlives one context: freed scratch stays mapped for the
 // next context or batch, so that a new one's first MSM does not wait for the
 // mapping (4 to 5 ms per GB).  At most SCRATCH_KEEP bytes per device stay,
@@ -144,7 +161,7 @@ void scratch_trim(int device) {
     std::lock_guard<std::mutex> g(g_pool_mu);
     auto it = g_pools.find(device);
     if (it == g_pools.end() || !it->second.pool) return;
-    cudaDeviceSynchronize();  // frees that are still in a stream
+    device_sync();  // frees that are still in a stream
     cudaMemPoolTrimTo(it->second.pool, 0);
 }
 
@@ -1340,7 +1357,7 @@ cudaError_t impeller_fail_scratch_step(uint32_t step) {
 cudaError_t impeller_ctx_destroy(impeller_ctx *ctx) {
     if (!ctx) return cudaSuccess;
     cudaSetDevice(ctx->device);
-    cudaDeviceSynchronize();
+    wait_idle(ctx->done);
     if (ctx->owns) cudaFree(const_cast<u32 *>(ctx->points));
     if (ctx->tables) cudaFree(ctx->tables);
     ctx->plans.clear();  // they hold images in the scratch pool
@@ -1363,7 +1380,7 @@ cudaError_t impeller_ctx_precompute(impeller_ctx *ctx, unsigned int c) {
     std::lock_guard<std::mutex> g(ctx->mu);
     if (ctx_set_base(ctx, c) != NONE) return cudaSuccess;
     CK(cudaSetDevice(ctx->device));
-    CK(cudaDeviceSynchronize());
+    CK(device_sync());
     const u32 W = digit_windows(c, ctx->curve);
     const u64 PB = (u64)point_words(ctx->curve) * 4, PW = point_words(ctx->curve);
     const u64 have = ctx->tables ? ctx->tables_points : ctx->len;  // region 0 = the points
@@ -1379,7 +1396,7 @@ cudaError_t impeller_ctx_precompute(impeller_ctx *ctx, unsigned int c) {
     u32 *set = t + (size_t)have * PW;
     if (e == cudaSuccess) e = cudaMemcpy(set, ctx->points, ctx->len * PB, cudaMemcpyDeviceToDevice);
     if (e == cudaSuccess) e = precompute_tables(set, ctx->len, c, W, 0, ctx->curve);
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = device_sync();
     if (e != cudaSuccess) {
         cudaFree(t);
         set_error(std::string("impeller_ctx_precompute: ") + cudaGetErrorString(e));
@@ -1388,7 +1405,7 @@ cudaError_t impeller_ctx_precompute(impeller_ctx *ctx, unsigned int c) {
     {
         std::unique_lock<std::shared_mutex> change(ctx->tables_mu);
         if (ctx->tables) {
-            cudaDeviceSynchronize();  // batches launched on them meanwhile
+            device_sync();  // batches launched on them meanwhile
             cudaFree(ctx->tables);
         }
         ctx->tables = t;
@@ -1527,6 +1544,7 @@ struct impeller_batch {
     cudaGraph_t g = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaStream_t cap_stream = nullptr;
+    cudaEvent_t done = nullptr;  // last run
     int device = 0;
     bool held = false;  // of the device's scratch pool
 };
@@ -1588,10 +1606,11 @@ cudaError_t impeller_batch_create(impeller_batch **out, impeller_ctx *ctx, const
 cudaError_t impeller_batch_destroy(impeller_batch *b) {
     if (!b) return cudaSuccess;
     cudaSetDevice(b->device);
-    cudaDeviceSynchronize();
+    wait_idle(b->done);
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->g) cudaGraphDestroy(b->g);
     if (b->cap_stream) cudaStreamDestroy(b->cap_stream);
+    if (b->done) cudaEventDestroy(b->done);
     if (b->scratch) cudaFreeAsync(b->scratch, nullptr);
     if (b->held) scratch_release(b->device);
     delete b;
@@ -1632,7 +1651,8 @@ cudaError_t impeller_batch_run(impeller_batch *b, const uint32_t *const *d_scala
         if (e != cudaSuccess) return e;
     } else {
         if (!b->exec) {
-            CK(cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking));
+            std::lock_guard<std::mutex> turn(g_capture_mu);
+            if (!b->cap_stream) CK(cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking));
             CK(cudaStreamBeginCapture(b->cap_stream, cudaStreamCaptureModeThreadLocal));
             e = b->plan.launch(b->scratch, ctx_point_base(b->ctx), nullptr, 0, b->cap_stream, nullptr, false);
             cudaGraph_t g = nullptr;
@@ -1649,6 +1669,8 @@ cudaError_t impeller_batch_run(impeller_batch *b, const uint32_t *const *d_scala
     CK(cudaMemcpyAsync(d_results, b->plan.results_ptr(b->scratch), (size_t)b->plan.M * point_words(b->plan.curve) * 4,
                        cudaMemcpyDeviceToDevice,
                        stream));
+    if (!b->done) CK(cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming));
+    CK(cudaEventRecord(b->done, stream));
     return cudaSuccess;
 }
 
